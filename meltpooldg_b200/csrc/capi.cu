@@ -257,12 +257,8 @@ mpdg_status mpdg_op_create(mpdg_mesh *mesh, const mpdg_op_desc *desc, mpdg_op **
     // 64^3 Q4 FP64 0.490 -> 0.485 ms; Q4 FP32 0.294 -> 0.299 ms, kept on warps)
     o.sched[MPDG_FP64].cta = (mm.degree == 2 || mm.degree == 4) ? 1 : 0;
     o.sched[MPDG_FP32].cta = mm.degree == 2 ? 1 : 0;
-    // the lane apply (uniform lattices, constant coefficients; other operators
-    // keep the warp apply) measured faster for Q2 on a B200: 128^3 advection-
-    // diffusion 0.664 -> 0.372 ms FP64, 0.431 -> 0.216 ms FP32; 64^3 heat
-    // 0.092 -> 0.052 ms FP64.  Below ~20^3 cells the warp apply is a little
-    // faster (16^3: 19.6 vs 20.5 us), so the default starts at 32^3 cells;
-    // the autotuner decides case by case.
+    // what the schedule reports where the band apply serves Q1/Q2; it runs by
+    // default on every lattice it serves, whatever the size and degree
     const int lane_default = (mm.degree == 2 && mm.n_cells >= 32768) ? 1 : 0;
     o.sched[MPDG_FP64].lane = lane_default;
     o.sched[MPDG_FP32].lane = lane_default;
@@ -485,6 +481,7 @@ mpdg_status mpdg_op_set_schedule(mpdg_op *op, int precision, const mpdg_schedule
     op->o.sched[precision].cta = sched->cta_cell_groups ? 1 : 0;
     if (sched->lane_cells < 0 || sched->lane_cells > 2) throw Error{MPDG_ERR_ARG, "lane_cells must be 0, 1 or 2"};
     op->o.sched[precision].lane = sched->lane_cells;
+    op->o.sched[precision].band = false;
     return MPDG_OK;
   });
 }

@@ -133,6 +133,7 @@ struct Mesh {
   bool has_dirichlet = false;
   size_t device_bytes = 0;
   bool metric32_ready = false;
+  int dirichlet_faces = 0;         // Dirichlet DoFs as whole box faces (bit 2 d + side; 0: not of that form)
   // Two-level mesh (hanging nodes): this mesh is the coarse block and `fine`
   // the fine block, refined 2:1 in y and z, meeting at the coarse block's
   // x = max face.  Vectors hold the coarse block's N_own DoFs, then the fine
@@ -174,7 +175,8 @@ struct ApplySchedule {
   int evict_first = 0;  // L2 evict-first hint on the coefficient stream
   int pdl = 1;          // colour launches as programmatic dependents of the previous one
   int cta = 0;          // cell groups of a whole CTA (Q2, Q4) instead of a warp
-  int lane = 0;         // one thread per cell (Q1, Q2 on uniform lattices, constant coefficients)
+  int lane = 0;         // Q1, Q2 on uniform lattices, constant coefficients: the band apply
+  bool band = true;     // the band apply wherever it serves the operator (off once a schedule is set)
 };
 
 struct Op {

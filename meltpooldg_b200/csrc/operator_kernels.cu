@@ -19,6 +19,7 @@
 #include <array>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "mpdg_internal.h"
@@ -595,7 +596,7 @@ __device__ __forceinline__ void law_eval(const KP<Real> &p, Real T, Real H, Real
 }
 
 #include "apply_warp.cuh"
-#include "apply_lane.cuh"
+#include "apply_band.cuh"
 #include "batch_apply.cuh"
 
 // ------------------------------------------------------------ the cell kernel
@@ -1606,6 +1607,36 @@ void build_mesh_device_data(Mesh &m, const uint8_t *host_mask, bool force_genera
       }
     }
     m.has_dirichlet = any;
+    // a mask that is a union of whole box faces (bit 2 d + side)
+    if (any) {
+      const long NXY = m.NX * m.NY;
+      auto face_of = [&](int f, long a, long b) {  // DoF (a, b) of face f
+        const int d = f / 2;
+        const long e = (f & 1) ? (d == 0 ? m.NX : d == 1 ? m.NY : m.NZ) - 1 : 0;
+        return d == 0 ? b * NXY + a * m.NX + e : d == 1 ? b * NXY + e * m.NX + a : e * NXY + b * m.NX + a;
+      };
+      int bits = 0;
+      for (int f = 0; f < 6; ++f) {
+        const long na = f / 2 == 0 ? m.NY : m.NX, nb = f / 2 == 2 ? m.NY : m.NZ;
+        bool all = true;
+        for (long b = 0; all && b < nb; ++b)
+          for (long a = 0; all && a < na; ++a) all = host_mask[face_of(f, a, b)] != 0;
+        if (all) bits |= 1 << f;
+      }
+      // (the bytes of such a mask are 0 or 1)
+      const std::vector<uint8_t> zeros(m.NX, 0), ones(m.NX, 1);
+      bool same = true;
+      for (long Z = 0; same && Z < m.NZ; ++Z)
+        for (long Y = 0; same && Y < m.NY; ++Y) {
+          const bool row = ((bits & 4) && Y == 0) || ((bits & 8) && Y == m.NY - 1) || ((bits & 16) && Z == 0) ||
+                           ((bits & 32) && Z == m.NZ - 1);
+          const uint8_t *r = host_mask + Z * NXY + Y * m.NX;
+          const uint8_t *in = row ? ones.data() : zeros.data();
+          same = (r[0] != 0) == (row || (bits & 1)) && (r[m.NX - 1] != 0) == (row || (bits & 2)) &&
+                 std::memcmp(r + 1, in, m.NX - 2) == 0;
+        }
+      if (same) m.dirichlet_faces = bits;
+    }
     if (any) {
       m.d_dmask = dev_alloc<uint8_t>(m.N, m.device_bytes);
       MPDG_CUDA(cudaMemcpy(m.d_dmask, host_mask, m.N, cudaMemcpyHostToDevice));
@@ -2111,121 +2142,179 @@ void run_warp_apply(Op &op, KP<Real> k)
   }
 }
 
-// the lane apply serves uniform lattices of degree 1 or 2 with one operand, no
-// hanging DoFs and a velocity it evaluates in-kernel
-template <typename Real>
-bool lane_apply_eligible(const Op &op, const KP<Real> &k)
+// the band apply serves uniform lattices with constant coefficients, no
+// hanging DoFs and a velocity that is a product along the axes.  The vortex
+// has (P+1)^2 coefficients of its own per x-unit; they are built for degrees 1
+// and 2.
+bool band_eligible(const Op &op)
 {
   const Mesh &m = *op.mesh;
-  return m.uniform && !m.mapped && (m.degree == 1 || m.degree == 2) && k.hsrc == nullptr &&
-         k.vel_kind != MPDG_VEL_NODAL;
+  if (!m.uniform || m.mapped || op.hang_src || supg(op) || uses_kT(op)) return false;
+  if (m.N >= (1L << 32) / 8) return false;  // 32-bit byte offsets
+  return op.d.vel_kind == MPDG_VEL_NONE || op.d.vel_kind == MPDG_VEL_CONST || op.d.vel_kind == MPDG_VEL_ROTATION ||
+         (op.d.vel_kind == MPDG_VEL_VORTEX && m.degree <= 2);
 }
 
-// the per-quadrature-point coefficient tables of the lane apply (degree P,
-// velocity kind VK) for the operator's constants
+// whether the schedule of one precision runs it: by default, and for degrees
+// 1 and 2 where lane_cells asks for it
+bool band_scheduled(const Op &op, int precision)
+{
+  const ApplySchedule &s = op.sched[precision];
+  return band_eligible(op) && (s.band || (s.lane && op.mesh->degree <= 2));
+}
+
+// element matrices of degree p on [0,1]: mass, stiffness, advection
+// (test function, derivative of the trial function), mass weighted by the coordinate
+struct LineMatrices {
+  double M[kMaxN * kMaxN], K[kMaxN * kMaxN], A[kMaxN * kMaxN], Mi[kMaxN * kMaxN];
+};
+const LineMatrices &line_matrices(int p)
+{
+  static const std::array<LineMatrices, kMaxDegree + 1> all = [] {
+    std::array<LineMatrices, kMaxDegree + 1> t{};
+    for (int p = 1; p <= kMaxDegree; ++p) {
+      const int n = p + 1;
+      double S[kMaxN * kMaxN], D[kMaxN * kMaxN], w[kMaxN], x[kMaxN];
+      shape_1d(p, S, D, w, x);
+      for (int i = 0; i < n; ++i)
+        for (int j = 0; j < n; ++j) {
+          double m = 0, k = 0, a = 0, mi = 0;
+          for (int q = 0; q < n; ++q) {
+            m += w[q] * S[q * n + i] * S[q * n + j];
+            k += w[q] * D[q * n + i] * D[q * n + j];
+            a += w[q] * S[q * n + i] * D[q * n + j];
+            mi += w[q] * x[q] * S[q * n + i] * S[q * n + j];
+          }
+          t[p].M[i * n + j] = m;
+          t[p].K[i * n + j] = k;
+          t[p].A[i * n + j] = a;
+          t[p].Mi[i * n + j] = mi;
+        }
+    }
+    return t;
+  }();
+  return all[p];
+}
+
 template <int P, typename Real, int VK>
-LaneCoef<Real> lane_coef(const KP<Real> &k)
+void run_band(Op &op, const KP<Real> &k)
 {
-  constexpr int n = P + 1, n2 = n * n, n3 = n2 * n;
-  double xq[kMaxN], wq[kMaxN], Dc[kMaxN * kMaxN];
-  gauss(n, xq, wq);
-  for (int q = 0; q < n; ++q)
-    for (int r = 0; r < n; ++r) {
-      double v, d;
-      lagrange(n, xq, r, xq[q], v, d);
-      Dc[q * n + r] = d;
-    }
-  const double hvol = (double)k.hvol;
-  double vf[3] = {1.0, 1.0, 1.0};  // the velocity factor the kernel does not evaluate
-  if (VK == LANE_VEL_CONST) for (int d = 0; d < 3; ++d) vf[d] = (double)k.vel_param[d];
-  if (VK == LANE_VEL_VORTEX) vf[1] = -1.0;
-  if (VK == LANE_VEL_ROTATION) vf[0] = (double)k.vel_param[0], vf[2] = -(double)k.vel_param[0];
-  LaneCoef<Real> c{};
-  for (int q = 0; q < n3; ++q) {
-    const double W = wq[q % n] * wq[(q / n) % n] * wq[q / n2];
-    c.mass[q] = (Real)((double)k.c_mass * hvol * W);
-    for (int d = 0; d < 3; ++d) {
-      c.diff[d][q] = (Real)((double)k.c_diff * hvol * (double)k.ih2[d] * W);
-      c.adv[d][q] = (Real)((double)k.c_vel * hvol * (double)k.ih[d] * W * vf[d]);
-    }
+  const Mesh &m = *op.mesh;
+  constexpr int n = P + 1, n2 = n * n;
+  using Real2 = typename Pair<Real>::type;
+  auto kern = band_apply_kernel<P, Real, VK>;
+  static const int regs = [&] {  // per instantiation
+    cudaFuncAttributes fa{};
+    MPDG_CUDA(cudaFuncGetAttributes(&fa, kern));
+    MPDG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
+    return std::max(16, fa.numRegs);
+  }();
+  BandP<P, Real> b{};
+  b.src = k.src;
+  b.dst = k.dst;
+  b.NX = m.NX;
+  b.NY = m.NY;
+  b.NZ = m.NZ;
+  for (int d = 0; d < 3; ++d) b.nc[d] = m.nc[d];
+  if (k.masked_read) {
+    b.faces = m.dirichlet_faces;
+    b.dmask = m.dirichlet_faces ? nullptr : m.d_dmask;
   }
-  for (int d = 0; d < 3; ++d)
-    for (int b = 0; b < n; ++b)
-      for (int a = 0; a < n; ++a) c.line[d][b * n + a] = (Real)((double)k.c_diff * hvol * (double)k.ih2[d] * wq[a] * wq[b]);
-  for (int r = 0; r < n; ++r)
-    for (int s = 0; s < n; ++s) {
-      double acc = 0.0;
-      for (int t = 0; t < n; ++t) acc += Dc[t * n + r] * wq[t] * Dc[t * n + s];
-      c.K[r * n + s] = (Real)acc;
-    }
-  return c;
-}
-
-template <int P, typename Real, int VK, int OCC>
-void run_lane_apply(Op &op, KP<Real> k)
-{
-  const LaneCoef<Real> coef = lane_coef<P, Real, VK>(k);
-  Mesh &m = *op.mesh;
-  if (m.N >= (1L << 32)) throw Error{MPDG_ERR_UNSUPPORTED, "the lane apply indexes DoFs with 32 bits"};
+  const LineMatrices &L = line_matrices(P);
+  const double cm = (double)k.c_mass, cv = (double)k.c_vel, cd = (double)k.c_diff;
+  const double *h = m.h, *u = op.d.vel_param;
+  const bool cst = op.d.vel_kind == MPDG_VEL_CONST;
+  const double vx = cst ? cv * u[0] : 0.0, vy = cst ? cv * u[1] : 0.0, vz = cst ? cv * u[2] : 0.0;
+  for (int e = 0; e < n2; ++e) {
+    b.Mx[e] = (Real)(h[0] * L.M[e]);
+    b.My[e] = (Real)(h[1] * L.M[e]);
+    b.Mz[e] = (Real)(h[2] * L.M[e]);
+    b.X1[e] = (Real)(cm * h[0] * L.M[e] + cd / h[0] * L.K[e] + vx * L.A[e]);
+    b.Y2[e] = (Real)(cd / h[1] * L.K[e] + vy * L.A[e]);
+    b.Z2[e] = (Real)(cd / h[2] * L.K[e] + vz * L.A[e]);
+    b.A[e] = (Real)L.A[e];
+    b.Mi[e] = (Real)L.Mi[e];
+  }
+  b.cv = (Real)(VK == BAND_ROTATION ? cv * u[0] : cv);
+  b.ox = (Real)m.origin[0];
+  b.oz = (Real)m.origin[2];
+  b.hx = (Real)h[0];
+  b.hy = (Real)h[1];
+  b.hz = (Real)h[2];
+  b.trig = k.trig;
+  b.trig_stride = k.trig_stride;
   constexpr int prec = sizeof(Real) == 4 ? MPDG_FP32 : MPDG_FP64;
-  const bool use_pdl = op.sched[prec].pdl != 0;
-  LaneColour lc{};
-  for (int c = 0; c < 8; ++c) {
-    lc.pfirst[c] = m.colour[c].first;
-    lc.pcn0[c] = m.colour[c].cn[0];
-    lc.pcn1[c] = m.colour[c].cn[1];
-  }
-  const int nseg = (m.nc[0] + kLaneSeg - 1) / kLaneSeg;
-  int launched = 0;
-  // the colour launches of cell layers [zlo, zhi) (all layers when empty), in
-  // the order x-segment parity, then y, then z parity
-  auto colour_launches = [&](int zlo, int zhi) {
-    for (int c = 0; c < 8; ++c) {
-      lc.sx = c & 1;
-      lc.py = (c >> 1) & 1;
-      lc.pz = (c >> 2) & 1;
-      lc.nsx = (nseg - lc.sx + 1) / 2;
-      lc.cny = (m.nc[1] - lc.py + 1) / 2;
-      const int zi0 = (zlo - lc.pz + 1) / 2, zi1 = (zhi - lc.pz + 1) / 2;
-      lc.zi0 = zi0;
-      lc.nwarps = (long)lc.nsx * lc.cny * std::max(0, zi1 - zi0);
-      if (lc.nwarps == 0) continue;
-      const bool pdl = use_pdl && launched > 0;
-      k.pdl = pdl ? 1 : 0;
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3((unsigned)((lc.nwarps + 3) / 4));
-      cfg.blockDim = dim3(128);
-      cfg.dynamicSmemBytes = 0;
-      cfg.stream = op.stream;
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-      attr[0].val.programmaticStreamSerializationAllowed = 1;
-      cfg.attrs = attr;
-      cfg.numAttrs = pdl ? 1 : 0;
-      MPDG_CUDA(cudaLaunchKernelEx(&cfg, lane_apply_kernel<P, Real, VK, OCC>, k, lc, coef));
-      MPDG_LAUNCHED();
-      ++launched;
+  using BS = BandShape<P, Real>;
+  // equal strips of at most the shape's x-units
+  const int ux = m.nc[0] + 1, uy = m.nc[1] + 1;
+  b.ntx = (ux + BS::nxu - 1) / BS::nxu;
+  b.nxu = (ux + b.ntx - 1) / b.ntx;
+  // fewer warps per CTA while the chip has CTAs to spare
+  b.warps = BS::warps;
+  while (b.warps > 1 && (long)b.ntx * ((uy + b.warps - 1) / b.warps) * m.nc[2] < num_sms()) b.warps /= 2;
+  b.nty = (uy + b.warps - 1) / b.warps;
+  constexpr size_t warp_smem = sizeof(Real2) * BS::warp_pairs(VK == BAND_VORTEX);
+  static_assert(warp_smem * BS::warps <= 160 * 1024, "shared memory set above");
+  const int threads = 32 * b.warps;
+  const size_t smem = warp_smem * b.warps;
+  const int per_sm = std::max(1, std::min({65536 / ((regs + 7) / 8 * 8 * threads), 2048 / threads, 32,
+                                           (int)((227 * 1024) / (smem + 1024))}));
+  const long resident = (long)num_sms() * per_sm;
+  auto layers = [&](int zlo, int zhi) {
+    b.zlo = zlo;
+    b.zhi = zhi;
+    // chunks of layers: few full waves, against the layer recomputed per chunk
+    const long tiles = (long)b.ntx * b.nty;
+    const int nz = zhi - zlo;
+    long best = -1;
+    for (int len = 1; len <= nz; ++len) {
+      const long chunks = (nz + len - 1) / len;
+      const long cost = ((tiles * chunks + resident - 1) / resident) * (len + (chunks > 1 || zlo > 0 ? 1 : 0));
+      if (best < 0 || cost <= best) {
+        best = cost;
+        b.len = len;
+      }
     }
+    const long grid = tiles * ((nz + b.len - 1) / b.len);
+    kern<<<(unsigned)grid, threads, smem, op.stream>>>(b);
+    MPDG_LAUNCHED();
   };
   if (k.zhi > k.zlo) {
-    colour_launches(k.zlo, k.zhi);
+    layers(k.zlo, k.zhi);
     return;
   }
-  // z-slabs with odd interior ends keep the first-touch rule across slabs
   int bounds[kMaxApplySlabs + 1];
   const int ns = slab_bounds(m.nc[2], apply_slabs(op, prec), bounds);
-  for (int sl = 0; sl < ns; ++sl) colour_launches(bounds[sl], bounds[sl + 1]);
+  for (int sl = 0; sl < ns; ++sl) layers(bounds[sl], bounds[sl + 1]);
 }
 
-template <int P, typename Real, int OCC>
-void lane_apply_velocity(Op &op, const KP<Real> &k)
+template <int P, typename Real>
+void band_apply_velocity(Op &op, const KP<Real> &k)
 {
-  switch (k.vel_kind) {
-    case MPDG_VEL_NONE: run_lane_apply<P, Real, LANE_VEL_NONE, OCC>(op, k); break;
-    case MPDG_VEL_CONST: run_lane_apply<P, Real, LANE_VEL_CONST, OCC>(op, k); break;
-    case MPDG_VEL_VORTEX: run_lane_apply<P, Real, LANE_VEL_VORTEX, OCC>(op, k); break;
-    case MPDG_VEL_ROTATION: run_lane_apply<P, Real, LANE_VEL_ROTATION, OCC>(op, k); break;
-    default: throw Error{MPDG_ERR_UNSUPPORTED, "velocity kind not evaluated by the lane apply"};
+  if (k.vel_kind == MPDG_VEL_ROTATION) {
+    run_band<P, Real, BAND_ROTATION>(op, k);
+  } else if (k.vel_kind == MPDG_VEL_VORTEX) {
+    if constexpr (P <= 2) run_band<P, Real, BAND_VORTEX>(op, k);
+  } else {
+    run_band<P, Real, BAND_PLAIN>(op, k);
+  }
+}
+
+template <typename Real>
+void band_apply(Op &op, const KP<Real> &k)
+{
+  // nothing is streamed per cell: several vectors go one after the other
+  for (int v = 0; v < std::max(1, k.nvec); ++v) {
+    KP<Real> kv = k;
+    kv.src = k.nvec > 1 ? k.msrc[v] : k.src;
+    kv.dst = k.nvec > 1 ? k.mdst[v] : k.dst;
+    switch (op.mesh->degree) {
+      case 1: band_apply_velocity<1, Real>(op, kv); break;
+      case 2: band_apply_velocity<2, Real>(op, kv); break;
+      case 3: band_apply_velocity<3, Real>(op, kv); break;
+      case 4: band_apply_velocity<4, Real>(op, kv); break;
+      default: throw Error{MPDG_ERR_UNSUPPORTED, "degree must be 1..4"};
+    }
   }
 }
 
@@ -2233,22 +2322,8 @@ template <typename Real, int GEOM>
 void warp_apply_degree(Op &op, const KP<Real> &k)
 {
   if constexpr (GEOM == GEOM_UNIFORM) {
-    const int lane = op.sched[sizeof(Real) == 4 ? MPDG_FP32 : MPDG_FP64].lane;
-    if (lane && lane_apply_eligible(op, k)) {
-      // a uniform lattice streams no coefficients, so a multi-vector apply
-      // loses nothing by applying its vectors in turn (and then returns the
-      // bits of the single applies)
-      for (int v = 0; v < std::max(1, k.nvec); ++v) {
-        KP<Real> kv = k;
-        kv.src = k.nvec > 1 ? k.msrc[v] : k.src;
-        kv.dst = k.nvec > 1 ? k.mdst[v] : k.dst;
-        kv.nvec = 1;
-        // Q1 fits either bound without spilling: one variant; lane 2 is the
-        // variant with more resident CTAs per SM
-        if (op.mesh->degree == 1) lane_apply_velocity<1, Real, 0>(op, kv);
-        else if (lane == 2) lane_apply_velocity<2, Real, 1>(op, kv);
-        else lane_apply_velocity<2, Real, 0>(op, kv);
-      }
+    if (band_scheduled(op, sizeof(Real) == 4 ? MPDG_FP32 : MPDG_FP64)) {
+      band_apply<Real>(op, k);
       return;
     }
   }
@@ -2837,19 +2912,21 @@ void autotune_apply(Op &op, int precision, int reps, ApplySchedule &best, double
   // candidates: slabs 1, 2, 4, 8, 16 (as many as the layers allow), each with and
   // without the evict-first hint where a coefficient stream exists
   std::vector<ApplySchedule> cand;
+  cand.push_back(op.sched[precision]);  // as the operator stands: by default the fastest known apply
   const bool stream = !m.uniform || m.mapped;
   const bool cta_differs = (m.degree == 2 || m.degree == 4) && !m.mapped && !op.fine;
   // the lane apply: uniform lattices of degree 1 or 2 whose vmult takes the
   // constant-coefficient path with an in-kernel velocity
   const bool lane_ok = m.uniform && !m.mapped && !op.fine && (m.degree == 1 || m.degree == 2) &&
                        plain_warp_apply(op) && !uses_kT(op) && op.d.vel_kind != MPDG_VEL_NODAL;
-  const int lane_max = lane_ok ? (m.degree == 2 ? 2 : 1) : 0;
+  const int lane_max = lane_ok && band_eligible(op) ? 1 : 0;
   for (int S : {1, 2}) {
     if (S > 1 && (S > m.nc[2] / 2 || m.mapped || op.fine)) continue;
     for (int h = 0; h <= (stream ? 1 : 0); ++h)
       for (int d = 0; d <= 1; ++d) {
         for (int g = 0; g <= (cta_differs ? 1 : 0); ++g) {
           ApplySchedule c;
+          c.band = false;
           c.slabs = S;
           c.evict_first = h;
           c.pdl = d;
@@ -2858,6 +2935,7 @@ void autotune_apply(Op &op, int precision, int reps, ApplySchedule &best, double
         }
         for (int l = 1; l <= lane_max; ++l) {
           ApplySchedule c;
+          c.band = false;
           c.slabs = S;
           c.evict_first = h;
           c.pdl = d;
