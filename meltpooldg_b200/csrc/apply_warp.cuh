@@ -339,11 +339,13 @@ __device__ __forceinline__ void l_backward(const Tables<Real> &T, Real *t0, Real
 // dynamic shared memory per cell group, in units of Real, rounded up to a
 // multiple of 8 elements so that every group's stage starts on a 32-byte
 // boundary (bulk copies need 16-byte aligned shared-memory destinations)
+// fluxes: the cell blocks of velocity values (1) or of velocity values and Newton
+// fluxes (2) beside the coefficients
 template <int P, typename Real, int GEOM, int GROUP = 32>
-__host__ __device__ constexpr int warp_smem_elems(bool vel)
+__host__ __device__ constexpr int warp_smem_elems(int fluxes)
 {
   constexpr int n = P + 1, CPW = GROUP / (n * n);
-  return (((GEOM == GEOM_GENERAL ? CPW * (metric_stride(n) + (vel ? velb_stride(n) : 0)) : 0) +
+  return (((GEOM == GEOM_GENERAL ? CPW * (metric_stride(n) + fluxes * velb_stride(n)) : 0) +
            TileLayout<n, Real, GROUP>::elems) + 7) / 8 * 8;
 }
 constexpr int kSmemAlign = 128;  // the dynamic shared-memory base is aligned by hand
@@ -376,8 +378,10 @@ struct WOcc {
 // GROUP: threads that share a group of cells -- 32 (a warp per group, four
 // groups per CTA) or 128 (the whole CTA per group, fewer idle lanes for Q2/Q4;
 // every tile exchange is then a CTA barrier)
+// NEWT: the velocity stream holds, per cell, the scaled velocity values (c_vel = 1)
+// and then the Newton flux, which adds its values times u to the flux
 template <int P, typename Real, int GEOM, bool HANG = false, bool MULTI = false, bool MAPPED = false,
-          int GROUP = 32>
+          int GROUP = 32, bool NEWT = false>
 __global__ void __launch_bounds__(kWarpsPerCTA * 32, WOcc<P, Real>::min_blocks)
     warp_apply_kernel(const KP<Real> p, int *err)
 {
@@ -385,17 +389,18 @@ __global__ void __launch_bounds__(kWarpsPerCTA * 32, WOcc<P, Real>::min_blocks)
   static_assert(!(MAPPED && (HANG || MULTI || GEOM != GEOM_GENERAL)), "mapped meshes: general geometry, one vector");
   static_assert(GROUP == 32 || (GROUP == kWarpsPerCTA * 32 && !HANG && !MULTI && !MAPPED),
                 "CTA-wide cell groups: plain applies only");
+  static_assert(!NEWT || (GEOM == GEOM_GENERAL && GROUP == 32 && !HANG && !MULTI && !MAPPED), "Newton flux: plain general applies");
   constexpr bool CTA = GROUP != 32;
   using L = TileLayout<P + 1, Real, GROUP>;
   constexpr int n = P + 1, n2 = n * n, n3 = n2 * n, CPW = GROUP / n2;
   constexpr int GPC = kWarpsPerCTA * 32 / GROUP;  // cell groups per CTA
-  constexpr int MS = metric_stride(n), VS = velb_stride(n);
+  constexpr int MS = metric_stride(n), VS = (NEWT ? 2 : 1) * velb_stride(n);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t bars[GPC];
   const Tables<Real> &T = tab<Real>(P);
   const int warp = CTA ? 0 : threadIdx.x >> 5, lane = CTA ? threadIdx.x : threadIdx.x & 31;
   const bool has_vel = p.vel_kind != MPDG_VEL_NONE;
-  const bool gvel = GEOM == GEOM_GENERAL && has_vel;
+  const bool gvel = GEOM == GEOM_GENERAL && (NEWT || has_vel);
 
   if (lane == 0) mbar_init(&bars[warp], 1);
   fence_mbar_init();
@@ -407,7 +412,7 @@ __global__ void __launch_bounds__(kWarpsPerCTA * 32, WOcc<P, Real>::min_blocks)
   bool dep_pending = p.pdl != 0;
 
   unsigned char *base = smem_raw + ((kSmemAlign - (smem_u32(smem_raw) & (kSmemAlign - 1))) & (kSmemAlign - 1));
-  Real *wsm = reinterpret_cast<Real *>(base) + warp * warp_smem_elems<P, Real, GEOM, GROUP>(gvel);
+  Real *wsm = reinterpret_cast<Real *>(base) + warp * warp_smem_elems<P, Real, GEOM, GROUP>(NEWT ? 2 : gvel ? 1 : 0);
   Real *stage = wsm;
   Real *vstage = wsm + (GEOM == GEOM_GENERAL ? CPW * MS : 0);
   Real *tiles = wsm + (GEOM == GEOM_GENERAL ? CPW * (MS + (gvel ? VS : 0)) : 0);
@@ -617,6 +622,12 @@ __global__ void __launch_bounds__(kWarpsPerCTA * 32, WOcc<P, Real>::min_blocks)
         fx[k] = G00 * gx[k] + G01 * gy[k] + G02 * gz[k];
         fy[k] = G01 * gx[k] + G11 * gy[k] + G12 * gz[k];
         fz[k] = G02 * gx[k] + G12 * gy[k] + G22 * gz[k];
+        if constexpr (NEWT) {
+          const Real *nf = vs + k * n2 + velb_stride(n);
+          fx[k] += nf[0] * uq[k];
+          fy[k] += nf[n3] * uq[k];
+          fz[k] += nf[2 * n3] * uq[k];
+        }
       } else {
         const Real JxW = p.hvol * T.w[i] * T.w[j] * T.w[k];
         if (nodal_vel) {

@@ -212,6 +212,11 @@ struct Op {
   double *d_coef64 = nullptr;
   float *d_coef32 = nullptr;
   bool coef64_ok = false, coef32_ok = false;
+  // operators whose coefficients follow the fields (phase laws, full tangent):
+  // per point c_vel JxW J^-1 u and the Newton flux dk/dT JxW J^-1 J^-T grad T
+  double *d_flux64 = nullptr;
+  float *d_flux32 = nullptr;
+  bool fields_frozen = false;  // inside a linear solve: the fields do not change
   size_t device_bytes = 0;
   // two-level mesh: the fine block's operator and the per-interface-cell stage
   // of the hanging DoFs' contributions to the coarse DoFs
@@ -313,6 +318,15 @@ inline bool law_has_solid(int mat) { return mat == MPDG_MAT_LIQUID_SOLID || mat 
 inline bool law_two_phase(int mat) { return mat == MPDG_MAT_GAS_LIQUID || mat == MPDG_MAT_GAS_LIQUID_SOLID; }
 // marks the merged coefficient stream stale (new temperature field or dt)
 void invalidate_coef(Op &op);
+// for the duration of a linear solve, in which the fields an operator reads are
+// constant: operators that otherwise read them in every apply merge them into
+// their coefficient streams once, from the fields as they are now
+struct FrozenFields {
+  Op &op;
+  bool was;
+  explicit FrozenFields(Op &o);
+  ~FrozenFields() { op.fields_frozen = was; }
+};
 
 template <typename Real>
 void launch_apply(Op &op, Real *dst, const Real *src);

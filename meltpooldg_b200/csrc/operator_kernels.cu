@@ -1108,6 +1108,97 @@ __global__ void __launch_bounds__(128) merge_kernel(const KP<double> p, const Co
   }
 }
 
+// the same for an operator whose coefficients follow the fields (k(T) on uniform
+// cells, the phase laws, the full Newton tangent): per point c_m JxW with the
+// Newton mass d(rho c_p)/dT ((T - T_old)/dt + u.grad T), k G, and (flux) c_v JxW
+// J^-1 u and the Newton flux dk/dT JxW J^-1 J^-T grad T -- the terms cell_kernel
+// evaluates in every apply.  Values are formed in FP64 and rounded once for the
+// FP32 form.
+template <int P, typename Real>
+__global__ void __launch_bounds__(128) field_merge_kernel(const KP<double> p, const ColourSet cs, long n_cells,
+                                                          Real *coef, Real *flux)
+{
+  constexpr int n = P + 1, n2 = n * n, n3 = n2 * n, CPB = Cfg<n>::cpb, MS = metric_stride(n), VS = velb_stride(n);
+  __shared__ double sm[CPB][n3];
+  __shared__ double sS[n2], sDc[n2];
+  const Tables<double> &T = tab<double>(P);
+  const int tid = threadIdx.x, slot = threadIdx.y;
+  const int i = tid % n, j = tid / n;
+  if (slot == 0) {
+    sS[tid] = T.S[tid];
+    sDc[tid] = T.Dc[tid];
+  }
+  __syncthreads();
+  const long cell = (long)blockIdx.x * CPB + slot;
+  const bool active = cell < n_cells;
+  int c = 0;
+  while (c < 7 && cell >= cs.c[c + 1].first) ++c;
+  const Colour &C = cs.c[c];
+  const long cidx = active ? cell - C.first : 0;
+  const int ix = active ? 2 * (int)(cidx % C.cn[0]) + C.par[0] : 0;
+  const int iy = active ? 2 * (int)((cidx / C.cn[0]) % C.cn[1]) + C.par[1] : 0;
+  const int iz = active ? 2 * (int)(cidx / ((long)C.cn[0] * C.cn[1])) + C.par[2] : 0;
+  const long zs = p.NX * p.NY;
+  const long g0 = ((long)(iz * P) * p.NY + (iy * P + j)) * p.NX + (ix * P + i);
+  double Tq[n], gx[n], gy[n], gz[n], Hq[n], Oq[n];
+  auto field = [&](const double *f, double (&q)[n]) {
+    double l[n];
+#pragma unroll
+    for (int k = 0; k < n; ++k) l[k] = f[g0 + k * zs];
+    to_qp<n>(sS, sm[slot], i, j, l, q);
+  };
+  field(p.T, Tq);
+  if (p.full_tangent) grad_qp<n>(sDc, sm[slot], i, j, Tq, gx, gy, gz);
+  if (p.Hs) field(p.Hs, Hq);
+  if (p.full_tangent && p.Told) field(p.Told, Oq);
+  if (!active) return;
+#pragma unroll
+  for (int k = 0; k < n; ++k) {
+    const int q = k * n2 + j * n + i;
+    double JxW, G[6] = {0, 0, 0, 0, 0, 0}, b[3] = {0, 0, 0};
+    if (p.metric) {
+      const double *m = p.metric + cell * MS + q;
+      JxW = m[0];
+#pragma unroll
+      for (int e = 0; e < 6; ++e) G[e] = m[(1 + e) * n3];
+    } else {
+      JxW = p.hvol * T.w[i] * T.w[j] * T.w[k];
+      G[0] = JxW * p.ih2[0];
+      G[3] = JxW * p.ih2[1];
+      G[5] = JxW * p.ih2[2];
+    }
+    if (p.velb) {
+      const double *vb = p.velb + cell * VS + q;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) b[d] = vb[d * n3];
+    } else if (p.vel_kind != MPDG_VEL_NONE) {
+      double uv[3];
+      uniform_velocity<double, n>(p, T, ix, iy, iz, i, j, k, uv);
+#pragma unroll
+      for (int d = 0; d < 3; ++d) b[d] = JxW * uv[d] * p.ih[d];
+    }
+    double cm, cv, kq, dcm, dcv, dk;
+    law_eval<double>(p, Tq[k], p.Hs ? Hq[k] : 0.0, cm, cv, kq, dcm, dcv, dk);
+    double mass = cm * JxW, f[3] = {0, 0, 0};
+    if (p.full_tangent) {
+      f[0] = dk * (G[0] * gx[k] + G[1] * gy[k] + G[2] * gz[k]);
+      f[1] = dk * (G[1] * gx[k] + G[3] * gy[k] + G[4] * gz[k]);
+      f[2] = dk * (G[2] * gx[k] + G[4] * gy[k] + G[5] * gz[k]);
+      if (p.Told) mass += dcm * (Tq[k] - Oq[k]) * JxW + dcv * (b[0] * gx[k] + b[1] * gy[k] + b[2] * gz[k]);
+    }
+    coef[cell * MS + q] = (Real)mass;
+#pragma unroll
+    for (int e = 0; e < 6; ++e) coef[cell * MS + (1 + e) * n3 + q] = (Real)(kq * G[e]);
+    if (flux) {
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        flux[cell * 2 * VS + d * n3 + q] = (Real)(cv * b[d]);
+        flux[cell * 2 * VS + VS + d * n3 + q] = (Real)f[d];
+      }
+    }
+  }
+}
+
 // ------------------------------------------------------ geometry kernels
 
 // per (cell, qp): JxW and G = JxW J^-1 J^-T of the trilinear map, colour-major
@@ -2053,13 +2144,14 @@ int num_sms()
   return g_num_sms;
 }
 
-template <int P, typename Real, int GEOM, bool HANG, bool MULTI = false, bool MAPPED = false, int GROUP = 32>
+template <int P, typename Real, int GEOM, bool HANG, bool MULTI = false, bool MAPPED = false, int GROUP = 32,
+          bool NEWT = false>
 void run_warp_apply(Op &op, KP<Real> k)
 {
   Mesh &m = *op.mesh;
   constexpr int n = P + 1, CPW = GROUP / (n * n), GPC = kWarpsPerCTA * 32 / GROUP;
-  const bool gvel = GEOM == GEOM_GENERAL && op.d.vel_kind != MPDG_VEL_NONE;
-  const size_t per_warp = sizeof(Real) * warp_smem_elems<P, Real, GEOM, GROUP>(gvel);
+  const bool gvel = GEOM == GEOM_GENERAL && (NEWT || op.d.vel_kind != MPDG_VEL_NONE);
+  const size_t per_warp = sizeof(Real) * warp_smem_elems<P, Real, GEOM, GROUP>(NEWT ? 2 : gvel ? 1 : 0);
   const size_t smem = per_warp * GPC + kSmemAlign;
   // bulk-copy alignment contract, checked before any launch: 16-byte aligned
   // shared destinations, global sources and sizes
@@ -2071,7 +2163,7 @@ void run_warp_apply(Op &op, KP<Real> k)
   if (GEOM == GEOM_GENERAL && (!k.metric || (gvel && !k.velb)))
     throw Error{MPDG_ERR_ARG, "coefficient stream missing"};
   if (m.N >= (1L << 32)) throw Error{MPDG_ERR_UNSUPPORTED, "the warp apply indexes DoFs with 32 bits"};
-  auto kern = warp_apply_kernel<P, Real, GEOM, HANG, MULTI, MAPPED, GROUP>;
+  auto kern = warp_apply_kernel<P, Real, GEOM, HANG, MULTI, MAPPED, GROUP, NEWT>;
   static int configured_smem = -1, blocks_per_sm = 0;  // per instantiation
   if (configured_smem != (int)smem) {
     MPDG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -2411,6 +2503,93 @@ void ensure_coef(Op &op, bool want32)
   op.coef32_ok = want32;
 }
 
+// operators whose apply reads the fields as they are now, not as they were at
+// mpdg_op_set_field: the block kernel evaluates them at the points in every apply.
+// In a linear solve, where they are constant, their terms are merged into the
+// warp apply's streams once (Q2, 30,720 cells, gas/liquid/solid law with velocity,
+// 46 applies of a Newton step's GMRES: 118 us per block apply, 67 us per warp
+// apply in eight launches one after the other, merge 46 us; step 7.0 -> 4.0 ms)
+bool live_fields(const Op &op)
+{
+  return uses_law(op) || (op.d.kind == MPDG_OP_HEAT && op.d.full_tangent) || (op.mesh->uniform && uses_kT(op));
+}
+
+// whether such an operator has velocity or Newton flux values beside the coefficients
+bool field_fluxes(const Op &op) { return uses_law(op) || op.d.full_tangent || op.d.vel_kind != MPDG_VEL_NONE; }
+
+template <typename Real>
+void ensure_field_coef(Op &op)
+{
+  Mesh &m = *op.mesh;
+  constexpr bool f32 = sizeof(Real) == 4;
+  bool &ok = f32 ? op.coef32_ok : op.coef64_ok;
+  if (ok) return;
+  const size_t count = (size_t)m.n_cells * metric_stride(m.n), fcount = 2 * (size_t)m.n_cells * velb_stride(m.n);
+  auto buffer = [&](auto *&p, size_t cnt) {  // padding is copied, never read
+    using R = std::remove_reference_t<decltype(*p)>;
+    if (p) return;
+    p = dev_alloc<R>(cnt, op.device_bytes);
+    MPDG_CUDA(cudaMemsetAsync(p, 0, sizeof(R) * cnt, op.stream));
+  };
+  Real *coef = nullptr, *flux = nullptr;
+  if constexpr (f32) {
+    buffer(op.d_coef32, count);
+    if (field_fluxes(op)) buffer(op.d_flux32, fcount);
+    coef = op.d_coef32;
+    flux = op.d_flux32;
+  } else {
+    buffer(op.d_coef64, count);
+    if (field_fluxes(op)) buffer(op.d_flux64, fcount);
+    coef = op.d_coef64;
+    flux = op.d_flux64;
+  }
+  KP<double> k = base_params<double>(op);
+  if (m.uniform) k.metric = nullptr;
+  ColourSet cs;
+  for (int c = 0; c < 8; ++c) cs.c[c] = m.colour[c];
+  auto run = [&](auto deg) {
+    constexpr int P = decltype(deg)::value, n = P + 1, CPB = Cfg<n>::cpb;
+    field_merge_kernel<P, Real><<<(unsigned)((m.n_cells + CPB - 1) / CPB), dim3(n * n, CPB), 0, op.stream>>>(
+        k, cs, m.n_cells, coef, flux);
+    MPDG_LAUNCHED();
+  };
+  switch (m.degree) {
+    case 1: run(std::integral_constant<int, 1>{}); break;
+    case 2: run(std::integral_constant<int, 2>{}); break;
+    case 3: run(std::integral_constant<int, 3>{}); break;
+    case 4: run(std::integral_constant<int, 4>{}); break;
+    default: throw Error{MPDG_ERR_UNSUPPORTED, "degree must be 1..4"};
+  }
+  ok = true;
+}
+
+template <typename Real>
+void frozen_field_apply(Op &op, KP<Real> k)
+{
+  ensure_field_coef<Real>(op);
+  const bool flux = field_fluxes(op);
+  if constexpr (sizeof(Real) == 8) {
+    k.metric = op.d_coef64;
+    if (flux) k.velb = op.d_flux64;
+  } else {
+    k.metric = op.d_coef32;
+    if (flux) k.velb = op.d_flux32;
+  }
+  k.c_vel = Real(1);
+  auto run = [&](auto deg) {
+    constexpr int P = decltype(deg)::value;
+    if (flux) run_warp_apply<P, Real, GEOM_GENERAL, false, false, false, 32, true>(op, k);
+    else run_warp_apply<P, Real, GEOM_GENERAL, false>(op, k);
+  };
+  switch (op.mesh->degree) {
+    case 1: run(std::integral_constant<int, 1>{}); break;
+    case 2: run(std::integral_constant<int, 2>{}); break;
+    case 3: run(std::integral_constant<int, 3>{}); break;
+    case 4: run(std::integral_constant<int, 4>{}); break;
+    default: throw Error{MPDG_ERR_UNSUPPORTED, "degree must be 1..4"};
+  }
+}
+
 }  // namespace
 
 // ---------------------------------------------------------- Robin boundary faces
@@ -2663,6 +2842,12 @@ void launch_robin(Op &op, Real *dst, const Real *src, int mode)
     }
 }
 
+FrozenFields::FrozenFields(Op &o) : op(o), was(o.fields_frozen)
+{
+  if (!was && live_fields(op)) op.coef64_ok = op.coef32_ok = false;
+  op.fields_frozen = true;
+}
+
 void invalidate_coef(Op &op)
 {
   op.coef64_ok = false;
@@ -2845,6 +3030,10 @@ void launch_cells(Op &op, Real *dst, const Real *src)
     return;
   }
   const bool law = uses_law(op);
+  if (op.fields_frozen && live_fields(op)) {
+    frozen_field_apply<Real>(op, k);
+    return;
+  }
   if (!full && !law && !m.uniform) {
     // general geometry: merged coefficient stream (k(T), c_mass, c_diff folded in)
     ensure_coef(op, sizeof(Real) == 4);

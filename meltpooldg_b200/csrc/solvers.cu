@@ -608,6 +608,7 @@ __global__ void cast_down_kernel(const double *a, float *b, long n)
 int solve(Op &op, const mpdg_solver_desc &d, double *x, const double *b, mpdg_solve_report &rep)
 {
   const auto t0 = std::chrono::steady_clock::now();
+  const FrozenFields frozen(op);
   Workspace &w = ws64(op);
   const long N = op.mesh->N;
   cudaStream_t s = op.stream;
