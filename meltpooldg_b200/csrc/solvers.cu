@@ -62,6 +62,7 @@ Workspace &ws64(Op &op)
     w.ct = walloc<double>(w, N);
     w.partial = walloc<double>(w, 128L * kRedBlocks);
     w.scal = walloc<double>(w, kNScalars + 128);
+    MPDG_CUDA(cudaMemsetAsync(w.scal, 0, sizeof(double) * kNScalars, op.stream));
     MPDG_CUDA(tracked_malloc_host(&w.host, sizeof(double) * (kNScalars + 128)));
   }
   return w;
@@ -149,9 +150,9 @@ int pcg(Op &op, Workspace &w, const Prec &P, const R *b, R *x, bool x_is_zero, d
     dev_axpby<R>(N, -1.0, v.Ap, 1.0, v.r, s);
   }
   if (sizeof(R) == 8)
-    dev_dot((const double *)v.r, (const double *)v.r, N, w.partial, sc + kRR, s);
+    dev_dot((const double *)v.r, (const double *)v.r, N, w.partial, sc + kRR, s, sc + kTICKET);
   else
-    dev_dot_f((const float *)v.r, (const float *)v.r, N, w.partial, sc + kRR, s);
+    dev_dot_f((const float *)v.r, (const float *)v.r, N, w.partial, sc + kRR, s, sc + kTICKET);
   res0 = std::sqrt(fetch(op, w, sc + kRR));
   res = res0;
   iters = 0;
@@ -161,15 +162,15 @@ int pcg(Op &op, Workspace &w, const Prec &P, const R *b, R *x, bool x_is_zero, d
   prec_apply<R>(op, P, v, v.r, v.z, applies);
   auto dot_into = [&](const R *a, const R *bb, double *out) {
     if (sizeof(R) == 8)
-      dev_dot((const double *)a, (const double *)bb, N, w.partial, out, s);
+      dev_dot((const double *)a, (const double *)bb, N, w.partial, out, s, sc + kTICKET);
     else
-      dev_dot_f((const float *)a, (const float *)bb, N, w.partial, out, s);
+      dev_dot_f((const float *)a, (const float *)bb, N, w.partial, out, s, sc + kTICKET);
   };
   dot_into(v.r, v.z, sc + kRZ);
   dev_copy<R>(N, v.z, v.p, s);
   const bool fused_jacobi = P.kind == MPDG_PREC_JACOBI;
   // The test |r| <= tol runs on the device after every iteration
-  // (dev_cg_check); the host reads its verdict every K iterations.  On small
+  // (in the update's last block); the host reads its verdict every K iterations.  On small
   // problems the round trip costs more than the iterations launched past
   // convergence, whose updates are skipped (x, r, p stay those of the
   // converged iteration: the result, the iteration count and the residual are
@@ -187,7 +188,6 @@ int pcg(Op &op, Workspace &w, const Prec &P, const R *b, R *x, bool x_is_zero, d
       launch_apply<R>(op, v.Ap, v.p);
       dot_into(v.p, v.Ap, sc + kPAP);
       dev_cg_update_lagged<R, R>(N, sc, x, v.r, v.p, v.Ap, fused_jacobi ? v.invd : nullptr, v.z, w.partial, s);
-      dev_cg_check(sc, s);
       if (!fused_jacobi) {
         int pa = 0;
         prec_apply<R>(op, P, v, v.r, v.z, pa);
@@ -295,7 +295,7 @@ int pcg_reliable(Op &op, Workspace &w, const Prec &P, const double *b, double *x
     ++applies;
     dev_copy<double>(N, b, w.r, s);
     dev_axpby<double>(N, -1.0, w.Ap, 1.0, w.r, s);
-    dev_dot(w.r, w.r, N, w.partial, sc + kRR, s);
+    dev_dot(w.r, w.r, N, w.partial, sc + kRR, s, sc + kTICKET);
     return std::sqrt(fetch(op, w, sc + kRR));
   };
   res0 = true_residual();
@@ -309,7 +309,7 @@ int pcg_reliable(Op &op, Workspace &w, const Prec &P, const double *b, double *x
   dev_scale_copy<float>(N, 1.0 / scale, w.r, v.r, s);
   auto precondition = [&]() {
     prec_apply<float>(op, P, v, v.r, v.z, applies);
-    dev_dot_f(v.r, v.z, N, w.partial, sc + kRZNEW, s);
+    dev_dot_f(v.r, v.z, N, w.partial, sc + kRZNEW, s, sc + kTICKET);
   };
   precondition();
   dev_copy<float>(N, v.z, v.p, s);
@@ -320,7 +320,7 @@ int pcg_reliable(Op &op, Workspace &w, const Prec &P, const double *b, double *x
   while (true) {
     launch_apply<float>(op, v.Ap, v.p);
     ++applies;
-    dev_dot_f(v.p, v.Ap, N, w.partial, sc + kPAP, s);
+    dev_dot_f(v.p, v.Ap, N, w.partial, sc + kPAP, s, sc + kTICKET);
     dev_cg_update<float, double>(N, sc, x, v.r, v.p, v.Ap, fused_jacobi ? v.invd : nullptr, v.z,
                                  w.partial, s, scale);
     ++iters;
@@ -555,14 +555,14 @@ double lanczos_lmax(Op &op, Workspace &w, int steps, int &applies)
   dev_copy<double>(N, start, r, s);
   dev_mul<double>(N, w.invd, r, z, s);
   dev_copy<double>(N, z, p, s);
-  dev_dot(r, z, N, w.partial, sc + kRZ, s);
+  dev_dot(r, z, N, w.partial, sc + kRZ, s, sc + kTICKET);
   std::vector<double> al, be;
   double *xdummy = w.ct;
   MPDG_CUDA(cudaMemsetAsync(xdummy, 0, sizeof(double) * N, s));
   for (int k = 0; k < steps; ++k) {
     launch_apply<double>(op, Ap, p);
     ++applies;
-    dev_dot(p, Ap, N, w.partial, sc + kPAP, s);
+    dev_dot(p, Ap, N, w.partial, sc + kPAP, s, sc + kTICKET);
     dev_cg_update<double, double>(N, sc, xdummy, r, p, Ap, w.invd, z, w.partial, s);
     MPDG_CUDA(cudaMemcpyAsync(w.host, sc, sizeof(double) * 4, cudaMemcpyDeviceToHost, s));
     MPDG_CUDA(cudaStreamSynchronize(s));
@@ -667,7 +667,7 @@ int solve(Op &op, const mpdg_solver_desc &d, double *x, const double *b, mpdg_so
     ++applies;
     dev_copy<double>(N, b, w.r, s);
     dev_axpby<double>(N, -1.0, w.Ap, 1.0, w.r, s);
-    dev_dot(w.r, w.r, N, w.partial, w.scal + kRR, s);
+    dev_dot(w.r, w.r, N, w.partial, w.scal + kRR, s, w.scal + kTICKET);
     res0 = std::sqrt(fetch(op, w, w.scal + kRR));
     res = res0;
     const double tol = std::fmax(abs_tol, rel * res0);
@@ -700,7 +700,7 @@ int solve(Op &op, const mpdg_solver_desc &d, double *x, const double *b, mpdg_so
       ++applies;
       dev_copy<double>(N, b, w.r, s);
       dev_axpby<double>(N, -1.0, w.Ap, 1.0, w.r, s);
-      dev_dot(w.r, w.r, N, w.partial, w.scal + kRR, s);
+      dev_dot(w.r, w.r, N, w.partial, w.scal + kRR, s, w.scal + kTICKET);
       res = std::sqrt(fetch(op, w, w.scal + kRR));
       ++outer;
       if (!std::isfinite(res)) status = MPDG_ERR_NAN;

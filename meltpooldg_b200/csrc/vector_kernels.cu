@@ -41,15 +41,41 @@ __device__ __forceinline__ double block_sum(double v)
   return s;
 }
 
+// True in the last block of the grid to get here: the blocks' partials written
+// before the call (by thread 0) are then visible to it.  The ticket counts the
+// blocks and is back at 0 afterwards; kernels of one stream may share it.  The last
+// block takes the place of a second launch that read the partials: at 36k DoFs a
+// CG iteration was 9 kernels of 2-4 us each and is 4 now.
+__device__ __forceinline__ bool last_block(double *ticket)
+{
+  __shared__ bool last;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicInc(reinterpret_cast<unsigned *>(ticket), gridDim.x - 1) == gridDim.x - 1;
+    __threadfence();
+  }
+  __syncthreads();
+  return last;
+}
+
+// sum of the grid's partials (valid in thread 0)
+__device__ __forceinline__ double partial_sum(const double *partial)
+{
+  double s = 0.0;
+  for (int i = threadIdx.x; i < (int)gridDim.x; i += kRedThreads) s += __ldcg(partial + i);
+  return block_sum(s);
+}
+
 // Grid-stride loops take kU elements per thread per pass (i, i + stride, ...,
 // loaded before any is used), so that each thread keeps kU loads of every
 // operand in flight; the per-thread order of a sum is the plain grid-stride
 // order, so reductions do not depend on kU.
 constexpr int kU = 4;
 
+// partials of a.b; with a ticket the last block adds them into *out
 template <typename A, typename B>
 __global__ void __launch_bounds__(kRedThreads) dot_partial_kernel(const A *a, const B *b, long n,
-                                                                  double *partial)
+                                                                  double *partial, double *ticket, double *out)
 {
   double s = 0.0;
   const long stride = (long)gridDim.x * blockDim.x;
@@ -68,6 +94,10 @@ __global__ void __launch_bounds__(kRedThreads) dot_partial_kernel(const A *a, co
   for (; i < n; i += stride) s += (double)a[i] * (double)b[i];
   s = block_sum(s);
   if (threadIdx.x == 0) partial[blockIdx.x] = s;
+  if (ticket && last_block(ticket)) {
+    const double t = partial_sum(partial);
+    if (threadIdx.x == 0) *out = t;
+  }
 }
 
 __global__ void __launch_bounds__(kRedThreads) linf_partial_kernel(const double *a, long n, double *partial)
@@ -246,10 +276,30 @@ __global__ void mul_kernel(long n, const R *d, const R *x, R *y)
     y[i] = d[i] * x[i];
 }
 
+// after each iteration: counts it (s[kCONV]) and runs the host loop's test
+// |r| <= tol (sqrt correctly rounded, so the decision is the host's) and the
+// non-finite check, once; r.r is kept, since later (skipped) iterations leave
+// the scalars alone.  The iteration number lives on the device, so a batch of
+// iterations is the same launch sequence every time (a graph replays it).
+__device__ __forceinline__ void cg_check(double *s)
+{
+  s[kCONV] += 1.0;
+  const double rr = s[kRR], res = sqrt(rr);
+  if (!isfinite(res)) {
+    s[kDONE] = 2.0;
+  } else if (res <= s[kTOL]) {
+    s[kDONE] = 1.0;
+  } else {
+    return;
+  }
+  s[kRRCONV] = rr;
+}
+
 // CG step part 1: alpha = s[RZ] / s[PAP]; x += alpha p; r -= alpha Ap;
-// with jacobi: z = invd r; partials of r.r (slot 0) and r.z (slot 1)
+// with jacobi: z = invd r; partials of r.r (slot 0) and r.z (slot 1), which the
+// last block adds into s[RR] and s[RZNEW]; it then (LAG) runs the convergence test
 template <typename R, typename RX, bool LAG = false>
-__global__ void __launch_bounds__(kRedThreads) cg_update_kernel(long n, const double *s, RX *x,
+__global__ void __launch_bounds__(kRedThreads) cg_update_kernel(long n, double *s, RX *x,
                                                                 R *r, const R *p, const R *Ap,
                                                                 const R *invd, R *z,
                                                                 double *partial, double xscale)
@@ -293,9 +343,17 @@ __global__ void __launch_bounds__(kRedThreads) cg_update_kernel(long n, const do
     rz = block_sum(rz);
     if (threadIdx.x == 0) partial[kRedBlocks + blockIdx.x] = rz;
   }
+  if (!last_block(s + kTICKET)) return;
+  rr = partial_sum(partial);
+  if (invd) rz = partial_sum(partial + kRedBlocks);
+  if (threadIdx.x == 0) {
+    s[kRR] = rr;
+    if (invd) s[kRZNEW] = rz;
+    if (LAG) cg_check(s);
+  }
 }
 
-// CG step part 2: beta = s[RZNEW] / s[RZ]; p = z + beta p; s[RZ] <- s[RZNEW] (block 0)
+// CG step part 2: beta = s[RZNEW] / s[RZ]; p = z + beta p; s[RZ] <- s[RZNEW] (last block)
 template <typename R, bool LAG = false>
 __global__ void cg_direction_kernel(long n, double *s, R *p, const R *z)
 {
@@ -314,36 +372,7 @@ __global__ void cg_direction_kernel(long n, double *s, R *p, const R *z)
     for (int u = 0; u < kU; ++u) p[i + u * stride] = (R)((double)vz[u] + beta * (double)vp[u]);
   }
   for (; i < n; i += stride) p[i] = (R)((double)z[i] + beta * (double)p[i]);
-}
-
-__global__ void shift_scalar_kernel(double *s)
-{
-  s[kRZ] = s[kRZNEW];
-}
-
-__global__ void shift_scalar_lagged_kernel(double *s)
-{
-  if (s[kDONE] == 0.0) s[kRZ] = s[kRZNEW];
-}
-
-// after each iteration: counts it (s[kCONV]) and runs the host loop's test
-// |r| <= tol (sqrt correctly rounded, so the decision is the host's) and the
-// non-finite check, once; r.r is kept, since later (skipped) iterations reuse
-// the partials.  The iteration number lives on the device, so a batch of
-// iterations is the same launch sequence every time (a graph replays it).
-__global__ void cg_check_kernel(double *s)
-{
-  if (s[kDONE] != 0.0) return;
-  s[kCONV] += 1.0;
-  const double rr = s[kRR], res = sqrt(rr);
-  if (!isfinite(res)) {
-    s[kDONE] = 2.0;
-  } else if (res <= s[kTOL]) {
-    s[kDONE] = 1.0;
-  } else {
-    return;
-  }
-  s[kRRCONV] = rr;
+  if (last_block(s + kTICKET) && threadIdx.x == 0) s[kRZ] = s[kRZNEW];
 }
 
 // Chebyshev start: d = invd r / theta; z = d
@@ -424,20 +453,30 @@ unsigned vgrid4(long n)
   if (g < 1) g = 1;
   return (unsigned)g;
 }
+// blocks of a reduction that its last block finishes: two elements per thread on
+// small vectors, where every block costs a ticket and a partial (36k DoFs: CG
+// update 12.7 us with 592 blocks, of which the last block's sums took 7)
+unsigned red_blocks(long n)
+{
+  const long g = (n + 2 * kRedThreads - 1) / (2 * kRedThreads);
+  return (unsigned)(g < 1 ? 1 : g > kRedBlocks ? kRedBlocks : g);
+}
 }  // namespace
 
-void dev_dot(const double *a, const double *b, long n, double *partial, double *out, cudaStream_t s)
+void dev_dot(const double *a, const double *b, long n, double *partial, double *out, cudaStream_t s, double *ticket)
 {
-  dot_partial_kernel<double, double><<<kRedBlocks, kRedThreads, 0, s>>>(a, b, n, partial);
+  dot_partial_kernel<double, double><<<ticket ? red_blocks(n) : kRedBlocks, kRedThreads, 0, s>>>(a, b, n, partial, ticket, out);
   MPDG_LAUNCHED();
+  if (ticket) return;
   finish_kernel<<<1, kRedThreads, 0, s>>>(partial, 1, out, 0);
   MPDG_LAUNCHED();
 }
 
-void dev_dot_f(const float *a, const float *b, long n, double *partial, double *out, cudaStream_t s)
+void dev_dot_f(const float *a, const float *b, long n, double *partial, double *out, cudaStream_t s, double *ticket)
 {
-  dot_partial_kernel<float, float><<<kRedBlocks, kRedThreads, 0, s>>>(a, b, n, partial);
+  dot_partial_kernel<float, float><<<ticket ? red_blocks(n) : kRedBlocks, kRedThreads, 0, s>>>(a, b, n, partial, ticket, out);
   MPDG_LAUNCHED();
+  if (ticket) return;
   finish_kernel<<<1, kRedThreads, 0, s>>>(partial, 1, out, 0);
   MPDG_LAUNCHED();
 }
@@ -531,16 +570,9 @@ template <typename R, typename RX>
 void dev_cg_update(long n, double *s, RX *x, R *r, const R *p, const R *Ap, const R *invd, R *z,
                    double *partial, cudaStream_t st, double xscale)
 {
-  cg_update_kernel<R, RX><<<kRedBlocks, kRedThreads, 0, st>>>(n, s, x, r, p, Ap, invd, z, partial,
+  cg_update_kernel<R, RX><<<red_blocks(n), kRedThreads, 0, st>>>(n, s, x, r, p, Ap, invd, z, partial,
                                                               xscale);
   MPDG_LAUNCHED();
-  // rr -> s[kRR]; rz -> s[kRZNEW]
-  finish_kernel<<<1, kRedThreads, 0, st>>>(partial, 1, s + kRR, 0);
-  MPDG_LAUNCHED();
-  if (invd) {
-    finish_kernel<<<1, kRedThreads, 0, st>>>(partial + kRedBlocks, 1, s + kRZNEW, 0);
-    MPDG_LAUNCHED();
-  }
 }
 template void dev_cg_update<double, double>(long, double *, double *, double *, const double *,
                                             const double *, const double *, double *, double *,
@@ -557,8 +589,6 @@ void dev_cg_direction(long n, double *s, R *p, const R *z, cudaStream_t st)
 {
   cg_direction_kernel<R><<<vgrid4(n), 256, 0, st>>>(n, s, p, z);
   MPDG_LAUNCHED();
-  shift_scalar_kernel<<<1, 1, 0, st>>>(s);
-  MPDG_LAUNCHED();
 }
 template void dev_cg_direction<double>(long, double *, double *, const double *, cudaStream_t);
 template void dev_cg_direction<float>(long, double *, float *, const float *, cudaStream_t);
@@ -567,14 +597,8 @@ template <typename R, typename RX>
 void dev_cg_update_lagged(long n, double *s, RX *x, R *r, const R *p, const R *Ap, const R *invd, R *z,
                           double *partial, cudaStream_t st)
 {
-  cg_update_kernel<R, RX, true><<<kRedBlocks, kRedThreads, 0, st>>>(n, s, x, r, p, Ap, invd, z, partial, 1.0);
+  cg_update_kernel<R, RX, true><<<red_blocks(n), kRedThreads, 0, st>>>(n, s, x, r, p, Ap, invd, z, partial, 1.0);
   MPDG_LAUNCHED();
-  finish_kernel<<<1, kRedThreads, 0, st>>>(partial, 1, s + kRR, 0);
-  MPDG_LAUNCHED();
-  if (invd) {
-    finish_kernel<<<1, kRedThreads, 0, st>>>(partial + kRedBlocks, 1, s + kRZNEW, 0);
-    MPDG_LAUNCHED();
-  }
 }
 template void dev_cg_update_lagged<double, double>(long, double *, double *, double *, const double *,
                                                    const double *, const double *, double *, double *,
@@ -587,8 +611,6 @@ template <typename R>
 void dev_cg_direction_lagged(long n, double *s, R *p, const R *z, cudaStream_t st)
 {
   cg_direction_kernel<R, true><<<vgrid4(n), 256, 0, st>>>(n, s, p, z);
-  MPDG_LAUNCHED();
-  shift_scalar_lagged_kernel<<<1, 1, 0, st>>>(s);
   MPDG_LAUNCHED();
 }
 template void dev_cg_direction_lagged<double>(long, double *, double *, const double *, cudaStream_t);
@@ -605,12 +627,6 @@ __global__ void cg_check_init_kernel(double *s, double tol)
 void dev_cg_check_init(double *s, double tol, cudaStream_t st)
 {
   cg_check_init_kernel<<<1, 1, 0, st>>>(s, tol);
-  MPDG_LAUNCHED();
-}
-
-void dev_cg_check(double *s, cudaStream_t st)
-{
-  cg_check_kernel<<<1, 1, 0, st>>>(s);
   MPDG_LAUNCHED();
 }
 
