@@ -87,8 +87,11 @@ struct BandP {
   static constexpr int n2 = (P + 1) * (P + 1);
   const Real *src;
   Real *dst;
-  const uint8_t *dmask;  // Dirichlet DoFs as bytes, or null
-  int faces;             // Dirichlet DoFs as whole box faces (bit 2 d + side)
+  // Dirichlet DoFs read as 0 and (w) not written: as whole box faces (bit 2 d +
+  // side), or as bytes, or none
+  const uint8_t *dmask, *wmask;
+  int faces, wfaces;
+  int add;               // adds to dst (constrained DoFs keep their value) instead of storing (0 there)
   long NX, NY, NZ;
   int nc[3];
   int nxu;               // x-units of a strip
@@ -140,6 +143,7 @@ __global__ void __launch_bounds__(BandShape<P, Real>::warps * 32) band_apply_ker
   const bool zero_hi0 = (yu == 0 && (p.faces & 4)) || (yu == p.nc[1] && (p.faces & 8));
   const bool zero_lo0 = yu == 1 && (p.faces & 4), zero_hiP = yu == p.nc[1] - 1 && (p.faces & 8);
   const bool inner = ylo && yhi && !zero_lo0 && !zero_hiP && !p.dmask;
+  const bool winner = ylo && yhi && !p.wmask && !p.add;
   const Real fyl = ylo ? Real(1) : Real(0), fyr = yhi ? Real(1) : Real(0);
   const unsigned rowb = (unsigned)p.NX * sizeof(Real), planeb = (unsigned)p.NY * rowb;
 
@@ -428,9 +432,9 @@ __global__ void __launch_bounds__(BandShape<P, Real>::warps * 32) band_apply_ker
         const int oc = lane + 32 * c, X = xb * P + oc;
         if (oc >= p.nxu * P || X >= (int)p.NX) continue;
         const unsigned o0 = (unsigned)(iz * P) * planeb + (unsigned)(yu * P) * rowb + (unsigned)X * (unsigned)sizeof(Real);
-        const bool ex = (X == 0 && (p.faces & 1)) || (X == (int)p.NX - 1 && (p.faces & 2));
-        const bool zfree = !(iz == 0 && (p.faces & 16)) && !top;
-        if (inner && zfree && !ex) {  // nothing constrained
+        const bool ex = (X == 0 && (p.wfaces & 1)) || (X == (int)p.NX - 1 && (p.wfaces & 2));
+        const bool zfree = !(iz == 0 && (p.wfaces & 16)) && !top;
+        if (winner && zfree && !ex) {  // nothing constrained
 #pragma unroll
           for (int k = 0; k < P; ++k) {
             unsigned o = o0 + (unsigned)k * planeb;
@@ -443,18 +447,78 @@ __global__ void __launch_bounds__(BandShape<P, Real>::warps * 32) band_apply_ker
         for (int k = 0; k < n; ++k) {
           if (k == P && !top) break;
           const int Z = iz * P + k;
-          const bool ez = (Z == 0 && (p.faces & 16)) || (Z == (int)p.NZ - 1 && (p.faces & 32));
+          const bool ez = (Z == 0 && (p.wfaces & 16)) || (Z == (int)p.NZ - 1 && (p.wfaces & 32));
           for (int i = 0; i < P; ++i) {
             if (i > 0 && !yhi) break;  // past the last vertex row
             const unsigned o = o0 + (unsigned)k * planeb + (unsigned)i * rowb;
-            bool masked = ex || ez || (i == 0 && zero_hi0);
-            if (p.dmask) masked = p.dmask[o / (unsigned)sizeof(Real)] != 0;
+            bool masked = ex || ez || (i == 0 && ((yu == 0 && (p.wfaces & 4)) || (yu == p.nc[1] && (p.wfaces & 8))));
+            if (p.wmask) masked = p.wmask[o / (unsigned)sizeof(Real)] != 0;
             const Real v = outs[k * BS::oplane + i * BS::orow + oc];
-            *reinterpret_cast<Real *>(reinterpret_cast<char *>(p.dst) + o) = masked ? Real(0) : v;
+            Real *d = reinterpret_cast<Real *>(reinterpret_cast<char *>(p.dst) + o);
+            if (p.add) *d += masked ? Real(0) : v;
+            else *d = masked ? Real(0) : v;
           }
         }
       }
       // staged again after at least one more __syncwarp
     }
+  }
+}
+
+// diagonal of the same operator: sums of products of the line matrices' diagonals
+// (a vertex has the last entry of the element before it and the first of its own).
+// Thread = column X of row blockIdx.y, marching along z.
+template <int P, typename Real, int VK>
+__global__ void __launch_bounds__(128) band_diag_kernel(const BandP<P, Real> p)
+{
+  constexpr int n = P + 1;
+  const Tables<Real> &T = tab<Real>(P);
+  const int X = blockIdx.x * blockDim.x + threadIdx.x, Y = blockIdx.y;
+  if (X >= (int)p.NX) return;
+  // f(element, local node) summed over the elements of line node `at`
+  auto line = [&](int at, int ne, auto f) -> Real {
+    const int e = at / P, i = at - e * P;
+    if (i > 0) return f(e, i);
+    return (e < ne ? f(e, 0) : Real(0)) + (e > 0 ? f(e - 1, P) : Real(0));
+  };
+  auto entry = [&](const Real *M) { return [=](int, int i) { return M[i * n + i]; }; };
+  // diagonal entries of mass and advection weighted by a function at the Gauss points
+  auto mass_of = [&](const Real *f, Real h) {
+    return [=](int e, int i) {
+      Real s = 0;
+      for (int q = 0; q < n; ++q) s += T.w[q] * f[e * n + q] * T.S[q * n + i] * T.S[q * n + i];
+      return h * s;
+    };
+  };
+  auto adv_of = [&](const Real *f) {
+    return [=](int e, int i) {
+      Real s = 0;
+      for (int q = 0; q < n; ++q) s += T.w[q] * f[e * n + q] * T.S[q * n + i] * T.D[q * n + i];
+      return s;
+    };
+  };
+  const int nx = p.nc[0], ny = p.nc[1], nz = p.nc[2];
+  const Real mx = line(X, nx, entry(p.Mx)), my = line(Y, ny, entry(p.My));
+  Real w = my * line(X, nx, entry(p.X1)) + line(Y, ny, entry(p.Y2)) * mx;  // times Mz
+  const Real v = my * mx;                                                 // times Z2
+  Real w2 = 0, v2 = 0;                                                    // rotation: times Mz(z) and Az
+  if constexpr (VK == BAND_VORTEX) {
+    const Real *tr = p.trig;
+    const int st = p.trig_stride;
+    w += p.cv * (line(Y, ny, mass_of(tr + 3 * st, p.hy)) * line(X, nx, adv_of(tr)) -
+                 line(Y, ny, adv_of(tr + 2 * st)) * line(X, nx, mass_of(tr + st, p.hx)));
+  }
+  if constexpr (VK == BAND_ROTATION) {
+    w2 = p.cv * my * line(X, nx, entry(p.A));
+    v2 = -p.cv * my * line(X, nx, [=](int e, int i) {
+      return (p.ox + e * p.hx) * p.Mx[i * n + i] + p.hx * p.hx * p.Mi[i * n + i];
+    });
+  }
+  for (int Z = blockIdx.z; Z < (int)p.NZ; Z += gridDim.z) {
+    Real d = line(Z, nz, entry(p.Mz)) * w + line(Z, nz, entry(p.Z2)) * v;
+    if constexpr (VK == BAND_ROTATION)
+      d += line(Z, nz, [=](int e, int i) { return (p.oz + e * p.hz) * p.Mz[i * n + i] + p.hz * p.hz * p.Mi[i * n + i]; }) * w2 +
+           line(Z, nz, entry(p.A)) * v2;
+    p.dst[((long)Z * p.NY + Y) * p.NX + X] = d;
   }
 }
