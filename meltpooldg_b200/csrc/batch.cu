@@ -98,8 +98,10 @@ struct Batch {
   double *d_adm = nullptr;   // admission scratch: reduction partials and |b|^2
   double *d_res = nullptr;   // result scratch of the copy stream
   BatchSchedule sched[3];    // heat slots, advection-diffusion slots, defect slots
-  cudaGraphExec_t graph = nullptr;
-  int64_t step_kernels = 0;  // kernels of one graph step
+  // step graphs: [0] while no advection-diffusion problem is resident (without
+  // that part's 26 kernels), [1] of both kinds; and their kernel counts
+  cudaGraphExec_t graph[2] = {nullptr, nullptr};
+  int64_t step_kernels[2] = {0, 0};
   BatchShape shape;          // block and tile shape of the batched FP32 apply (autotuned)
   double tuned_ms = 0;
   double *d_norms = nullptr;  // |x|^2 of finished slots (serving)
@@ -450,9 +452,40 @@ __device__ double slot_sum(const BatchTables &T, int s)
 {
   const double *p = T.part[s];
   const int nc = T.info[s].n_chunks;
+  // 32 loads in flight (one thread per slot: a load at a time took 15-24 us per
+  // sum of a 1.4 M-DoF problem's 170 chunks, 3 us so), summed in chunk order
+  constexpr int U = 32;
   double v = 0.0;
-  for (int c = 0; c < nc; ++c) v += p[4 * c + K];
+  int c = 0;
+  for (; c + U <= nc; c += U) {
+    double t[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) t[u] = p[4 * (c + u) + K];
+#pragma unroll
+    for (int u = 0; u < U; ++u) v += t[u];
+  }
+#pragma unroll 8
+  for (; c < nc; ++c) v += p[4 * c + K];
   return v;
+}
+
+// f(i, values of the operands at i) for a chunk's elements of this thread, kBU
+// elements loaded before any is stored (a store may alias the next load), in the
+// order of the plain strided loop: sums keep their bits
+constexpr int kBU = 4;
+template <typename L, typename F>
+__device__ __forceinline__ void chunk_loop(long begin, long end, L load, F f)
+{
+  const int bd = blockDim.x;
+  long i = begin + threadIdx.x;
+  for (; i + (kBU - 1) * bd < end; i += kBU * bd) {
+    decltype(load(i)) v[kBU];
+#pragma unroll
+    for (int u = 0; u < kBU; ++u) v[u] = load(i + u * bd);
+#pragma unroll
+    for (int u = 0; u < kBU; ++u) f(i + u * bd, v[u]);
+  }
+  for (; i < end; i += bd) f(i, load(i));
 }
 
 // ------------------------------------------------------ CG (heat problems)
@@ -464,7 +497,10 @@ __global__ void bk_dot_pap(BatchSchedule S, BatchTables T, const int *active)
     double d = 0.0;
     if (active[s]) {
       const float *a = T.p[s], *b = T.Ap[s];
-      for (long i = begin + threadIdx.x; i < end; i += blockDim.x) d += (double)a[i] * (double)b[i];
+      struct V {
+        float a, b;
+      };
+      chunk_loop(begin, end, [=](long i) { return V{a[i], b[i]}; }, [&](long, const V &v) { d += (double)v.a * (double)v.b; });
     }
     d = bblock_sum(d);
     if (threadIdx.x == 0) part[0] = d;
@@ -488,15 +524,20 @@ __global__ void bk_cg_update(BatchSchedule S, BatchTables T, const int *active, 
       double *x = T.x[s];
       float *r = T.r[s], *z = T.z[s];
       const float *p = T.p[s], *ap = T.Ap[s], *id = T.invd[s];
-      for (long i = begin + threadIdx.x; i < end; i += blockDim.x) {
-        x[i] += xa * (double)p[i];
-        const float ri = (float)((double)r[i] - alpha * (double)ap[i]);
-        r[i] = ri;
-        const float zi = id[i] * ri;
-        z[i] = zi;
-        rr += (double)ri * (double)ri;
-        rz += (double)ri * (double)zi;
-      }
+      struct V {
+        double x;
+        float p, r, ap, id;
+      };
+      chunk_loop(begin, end, [=](long i) { return V{x[i], p[i], r[i], ap[i], id[i]}; },
+                 [&](long i, const V &v) {
+                   x[i] = v.x + xa * (double)v.p;
+                   const float ri = (float)((double)v.r - alpha * (double)v.ap);
+                   r[i] = ri;
+                   const float zi = v.id * ri;
+                   z[i] = zi;
+                   rr += (double)ri * (double)ri;
+                   rz += (double)ri * (double)zi;
+                 });
     }
     rr = bblock_sum(rr);
     rz = bblock_sum(rz);
@@ -542,11 +583,15 @@ __global__ void bk_defect(BatchSchedule S, BatchTables T, const int *defect)
     if (defect[s]) {
       const double *b = T.b[s];
       double *r = T.r64[s];
-      for (long i = begin + threadIdx.x; i < end; i += blockDim.x) {
-        const double d = b[i] - r[i];
-        r[i] = d;
-        d2 += d * d;
-      }
+      struct V {
+        double b, r;
+      };
+      chunk_loop(begin, end, [=](long i) { return V{b[i], r[i]}; },
+                 [&](long i, const V &v) {
+                   const double d = v.b - v.r;
+                   r[i] = d;
+                   d2 += d * d;
+                 });
     }
     d2 = bblock_sum(d2);
     if (threadIdx.x == 0) part[3] = d2;
@@ -587,13 +632,18 @@ __global__ void bk_cg_replace(BatchSchedule S, BatchTables T, const int *defect,
       const double *d = T.r64[s];
       float *r = T.r[s], *z = T.z[s];
       const float *id = T.invd[s];
-      for (long i = begin + threadIdx.x; i < end; i += blockDim.x) {
-        const float ri = (float)(d[i] * is);
-        r[i] = ri;
-        const float zi = id[i] * ri;
-        z[i] = zi;
-        rz += (double)ri * (double)zi;
-      }
+      struct V {
+        double d;
+        float id;
+      };
+      chunk_loop(begin, end, [=](long i) { return V{d[i], id[i]}; },
+                 [&](long i, const V &v) {
+                   const float ri = (float)(v.d * is);
+                   r[i] = ri;
+                   const float zi = v.id * ri;
+                   z[i] = zi;
+                   rz += (double)ri * (double)zi;
+                 });
     }
     rz = bblock_sum(rz);
     if (threadIdx.x == 0) part[2] = rz;
@@ -615,7 +665,11 @@ __global__ void bk_cg_direction(BatchSchedule S, BatchTables T, const int *activ
       const double beta = sc[s].rz_new / sc[s].rz;
       const float *z = T.z[s];
       float *p = T.p[s];
-      for (long i = begin + threadIdx.x; i < end; i += blockDim.x) p[i] = (float)((double)z[i] + beta * (double)p[i]);
+      struct V {
+        float z, p;
+      };
+      chunk_loop(begin, end, [=](long i) { return V{z[i], p[i]}; },
+                 [&](long i, const V &v) { p[i] = (float)((double)v.z + beta * (double)v.p); });
     }
   END_FOR_CHUNK
 }
@@ -1013,14 +1067,14 @@ void free_schedule(BatchSchedule &S)
 
 void drop_graph(Batch &B)
 {
-  if (B.graph) {
-    cudaGraphExecDestroy(B.graph);
-    B.graph = nullptr;
+  for (auto &g : B.graph) {
+    if (g) cudaGraphExecDestroy(g);
+    g = nullptr;
   }
 }
 
 // one Krylov step of every running slot (the body of the graph)
-void enqueue_step(Batch &B, const BatchShape &shape)
+void enqueue_step(Batch &B, const BatchShape &shape, bool advdiff)
 {
   const BatchShape shape64;  // the FP64 defect applies (a few per solve) keep the default shape
   cudaStream_t st = B.stream;
@@ -1035,8 +1089,10 @@ void enqueue_step(Batch &B, const BatchShape &shape)
   } while (0)
   bk_schedule<<<9, kSchedThreads, 0, st>>>(B.d_active, MPDG_OP_HEAT, T.info, S, SH);
   MPDG_LAUNCHED();
-  bk_schedule<<<9, kSchedThreads, 0, st>>>(B.d_active, MPDG_OP_ADVDIFF, T.info, S, SA);
-  MPDG_LAUNCHED();
+  if (advdiff) {
+    bk_schedule<<<9, kSchedThreads, 0, st>>>(B.d_active, MPDG_OP_ADVDIFF, T.info, S, SA);
+    MPDG_LAUNCHED();
+  }
   // CG on the heat problems: Ap = A p (FP32), alpha, x/r/z update
   launch_batch_apply<float>(SH, T.info, B.d_params, T.p, T.Ap, B.d_active, shape, st);
   BK(bk_dot_pap, gc, SH, T, B.d_active);
@@ -1044,16 +1100,18 @@ void enqueue_step(Batch &B, const BatchShape &shape)
   BK(bk_cg_update, gc, SH, T, B.d_active, B.d_sc);
   BK(bk_cg_decide, gs, B.d_sc, B.d_active, B.d_defect, T, S, B.delta);
   // BiCGStab on the advection-diffusion problems: v = A M p, alpha, s, t = A M s, omega, update
-  BK(bk_bicg_precond_p, gc, SA, T, B.d_active, B.d_sc);
-  launch_batch_apply<float>(SA, T.info, B.d_params, T.z, T.v, B.d_active, shape, st);
-  BK(bk_bicg_alpha_partials, gc, SA, T, B.d_active, B.d_sc);
-  BK(bk_bicg_alpha, gs, B.d_sc, B.d_active, T, S);
-  BK(bk_bicg_s, gc, SA, T, B.d_active, B.d_sc);
-  launch_batch_apply<float>(SA, T.info, B.d_params, T.z, T.t, B.d_active, shape, st);
-  BK(bk_bicg_omega_partials, gc, SA, T, B.d_active, B.d_sc);
-  BK(bk_bicg_omega, gs, B.d_sc, B.d_active, T, S);
-  BK(bk_bicg_update, gc, SA, T, B.d_active, B.d_sc);
-  BK(bk_bicg_decide, gs, B.d_sc, B.d_active, B.d_defect, T, S, B.delta);
+  if (advdiff) {
+    BK(bk_bicg_precond_p, gc, SA, T, B.d_active, B.d_sc);
+    launch_batch_apply<float>(SA, T.info, B.d_params, T.z, T.v, B.d_active, shape, st);
+    BK(bk_bicg_alpha_partials, gc, SA, T, B.d_active, B.d_sc);
+    BK(bk_bicg_alpha, gs, B.d_sc, B.d_active, T, S);
+    BK(bk_bicg_s, gc, SA, T, B.d_active, B.d_sc);
+    launch_batch_apply<float>(SA, T.info, B.d_params, T.z, T.t, B.d_active, shape, st);
+    BK(bk_bicg_omega_partials, gc, SA, T, B.d_active, B.d_sc);
+    BK(bk_bicg_omega, gs, B.d_sc, B.d_active, T, S);
+    BK(bk_bicg_update, gc, SA, T, B.d_active, B.d_sc);
+    BK(bk_bicg_decide, gs, B.d_sc, B.d_active, B.d_defect, T, S, B.delta);
+  }
   // FP64 defects b - A x of the slots whose FP32 residual dropped by delta (or that look converged)
   bk_schedule<<<9, kSchedThreads, 0, st>>>(B.d_defect, -1, T.info, S, SD);
   MPDG_LAUNCHED();
@@ -1062,28 +1120,32 @@ void enqueue_step(Batch &B, const BatchShape &shape)
   BK(bk_defect_decide, gs, B.d_sc, B.d_active, B.d_defect, T, S);
   BK(bk_cg_replace, gc, SD, T, B.d_defect, B.d_sc);
   BK(bk_cg_replace_finish, gs, B.d_sc, B.d_defect, T, S);
-  BK(bk_bicg_replace, gc, SD, T, B.d_defect, B.d_sc);
-  BK(bk_bicg_replace_finish, gs, B.d_sc, B.d_defect, T, S);
+  if (advdiff) {
+    BK(bk_bicg_replace, gc, SD, T, B.d_defect, B.d_sc);
+    BK(bk_bicg_replace_finish, gs, B.d_sc, B.d_defect, T, S);
+  }
   // search directions and scalar shifts
   BK(bk_cg_direction, gc, SH, T, B.d_active, B.d_sc);
-  BK(bk_bicg_direction, gc, SA, T, B.d_active, B.d_defect, B.d_sc);
   BK(bk_cg_shift, gs, B.d_sc, B.d_active, S);
-  BK(bk_bicg_shift, gs, B.d_sc, B.d_active, S);
+  if (advdiff) {
+    BK(bk_bicg_direction, gc, SA, T, B.d_active, B.d_defect, B.d_sc);
+    BK(bk_bicg_shift, gs, B.d_sc, B.d_active, S);
+  }
   BK(bk_count_running, 1, B.d_active, S, B.d_running);
 #undef BK
 }
 
-// the step graph; independent of the slots in use, so captured once (again
+// the step graphs; independent of the slots in use, so captured once (again
 // only when the autotuner changes the apply's grid)
-void ensure_graph(Batch &B)
+void ensure_graph(Batch &B, int which)
 {
-  if (B.graph) return;
+  if (B.graph[which]) return;
   batch_apply_setup();  // set-up of the launchers outside the capture
   const int64_t before = mpdg_kernel_launches();
   cudaGraph_t g = nullptr;
   MPDG_CUDA(cudaStreamBeginCapture(B.stream, cudaStreamCaptureModeThreadLocal));
   try {
-    enqueue_step(B, B.shape);
+    enqueue_step(B, B.shape, which == 1);
   } catch (...) {
     cudaStreamEndCapture(B.stream, &g);
     if (g) cudaGraphDestroy(g);
@@ -1091,12 +1153,12 @@ void ensure_graph(Batch &B)
     throw;
   }
   MPDG_CUDA(cudaStreamEndCapture(B.stream, &g));
-  B.step_kernels = mpdg_kernel_launches() - before;
-  count_launch(-(int)B.step_kernels);  // captured, not launched
-  const cudaError_t e = cudaGraphInstantiate(&B.graph, g, 0);
+  B.step_kernels[which] = mpdg_kernel_launches() - before;
+  count_launch(-(int)B.step_kernels[which]);  // captured, not launched
+  const cudaError_t e = cudaGraphInstantiate(&B.graph[which], g, 0);
   cudaGraphDestroy(g);
   if (e != cudaSuccess) {
-    B.graph = nullptr;
+    B.graph[which] = nullptr;
     throw Error{MPDG_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e)};
   }
 }
@@ -1224,9 +1286,11 @@ void report_of(const SlotScalars &q, mpdg_solve_report &rep)
 
 void launch_steps(Batch &B, int k)
 {
-  ensure_graph(B);
-  for (int i = 0; i < k; ++i) MPDG_CUDA(cudaGraphLaunch(B.graph, B.stream));
-  count_launch((int)(k * B.step_kernels));
+  int which = 0;
+  for (const BatchSlot &S : B.slots) which |= S.used && S.desc.kind == MPDG_OP_ADVDIFF;
+  ensure_graph(B, which);
+  for (int i = 0; i < k; ++i) MPDG_CUDA(cudaGraphLaunch(B.graph[which], B.stream));
+  count_launch((int)(k * B.step_kernels[which]));
 }
 
 // up to max_steps graph launches, reading the running count every poll steps
