@@ -362,6 +362,65 @@ __device__ __forceinline__ void colour_cell(int cidx, const KPT &p, int &ix, int
   iz = 2 * (int)q01 + p.par[2];
 }
 
+// the colours of a lattice as runs of warp groups in one launch: groups[c] is the
+// first group of colour c, groups[8] their number
+struct ColourRuns {
+  int groups[9], count[8], cn0[8], cn1[8];
+  long first[8];
+  unsigned long long m0[8], m01[8];  // magic divisors of cn0 and cn0 cn1 (KP::div0_magic)
+  __device__ __forceinline__ void cell(int c, int cidx, int &ix, int &iy, int &iz) const
+  {
+    const unsigned x = (unsigned)cidx;
+    const unsigned q0 = (unsigned)(((unsigned long long)x * m0[c]) >> 40);
+    const unsigned q01 = (unsigned)(((unsigned long long)x * m01[c]) >> 40);
+    ix = 2 * (int)(x - q0 * (unsigned)cn0[c]) + (c & 1);
+    iy = 2 * (int)(q0 - q01 * (unsigned)cn1[c]) + ((c >> 1) & 1);
+    iz = 2 * (int)q01 + (c >> 2);
+  }
+};
+
+// dst from the cells' local results: a DoF adds the values of its cells in the order
+// of their colours, as the coloured launches do, so the bits are the same;
+// constrained DoFs get 0
+template <int P, typename Real>
+__global__ void __launch_bounds__(128) local_gather_kernel(const KP<Real> p, const ColourRuns runs)
+{
+  constexpr int n = P + 1, n2 = n * n, n3 = n2 * n;
+  const int X = blockIdx.x * blockDim.x + threadIdx.x, Y = blockIdx.y, Z = blockIdx.z;
+  const bool in = X < (int)p.NX;
+  const long g = ((long)Z * p.NY + Y) * p.NX + (in ? X : 0);
+  const bool masked = in && p.masked_write && p.dmask && p.dmask[g];
+  // per axis and parity: the cell of that parity that has the node, and the node in it
+  int cx[2], lx[2], cy[2], ly[2], cz[2], lz[2];
+  auto axis = [](int at, int nc, int (&c)[2], int (&l)[2]) {
+    const int e = at / P, i = at - e * P;
+    c[0] = c[1] = -1;
+    l[0] = l[1] = 0;
+    if (e < nc) {
+      c[e & 1] = e;
+      l[e & 1] = i;
+    }
+    if (i == 0 && e > 0) {
+      c[(e - 1) & 1] = e - 1;
+      l[(e - 1) & 1] = P;
+    }
+  };
+  axis(X, p.nc[0], cx, lx);
+  axis(Y, p.nc[1], cy, ly);
+  axis(Z, p.nc[2], cz, lz);
+  grid_dep_wait();
+  if (!in) return;
+  Real s = 0;
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    const int a = c & 1, b = (c >> 1) & 1, d = c >> 2;
+    if (cx[a] < 0 || cy[b] < 0 || cz[d] < 0) continue;
+    const long cell = runs.first[c] + ((long)(cz[d] >> 1) * runs.cn1[c] + (cy[b] >> 1)) * runs.cn0[c] + (cx[a] >> 1);
+    s += __ldcg(p.local + cell * n3 + lz[d] * n2 + ly[b] * n + lx[a]);
+  }
+  p.dst[g] = masked ? Real(0) : s;
+}
+
 template <int P, typename Real>
 struct WOcc {
   static constexpr int min_blocks = (sizeof(Real) == 8) ? (P == 4 ? 3 : P == 3 ? 4 : P == 2 ? 5 : 6)
@@ -380,16 +439,19 @@ struct WOcc {
 // every tile exchange is then a CTA barrier)
 // NEWT: the velocity stream holds, per cell, the scaled velocity values (c_vel = 1)
 // and then the Newton flux, which adds its values times u to the flux
+// LOCAL: all colours in one launch; a cell's results go to its n^3 values of p.local
+// (colour-major), which local_gather_kernel adds per DoF in colour order
 template <int P, typename Real, int GEOM, bool HANG = false, bool MULTI = false, bool MAPPED = false,
-          int GROUP = 32, bool NEWT = false>
+          int GROUP = 32, bool NEWT = false, bool LOCAL = false>
 __global__ void __launch_bounds__(kWarpsPerCTA * 32, WOcc<P, Real>::min_blocks)
-    warp_apply_kernel(const KP<Real> p, int *err)
+    warp_apply_kernel(const KP<Real> p, int *err, const ColourRuns runs)
 {
   static_assert(!(HANG && MULTI), "the multi-vector apply has no hanging-node path");
   static_assert(!(MAPPED && (HANG || MULTI || GEOM != GEOM_GENERAL)), "mapped meshes: general geometry, one vector");
   static_assert(GROUP == 32 || (GROUP == kWarpsPerCTA * 32 && !HANG && !MULTI && !MAPPED),
                 "CTA-wide cell groups: plain applies only");
   static_assert(!NEWT || (GEOM == GEOM_GENERAL && GROUP == 32 && !HANG && !MULTI && !MAPPED), "Newton flux: plain general applies");
+  static_assert(!LOCAL || (GROUP == 32 && !HANG && !MULTI && !MAPPED), "local results: plain applies");
   constexpr bool CTA = GROUP != 32;
   using L = TileLayout<P + 1, Real, GROUP>;
   constexpr int n = P + 1, n2 = n * n, n3 = n2 * n, CPW = GROUP / n2;
@@ -406,10 +468,10 @@ __global__ void __launch_bounds__(kWarpsPerCTA * 32, WOcc<P, Real>::min_blocks)
   fence_mbar_init();
   __syncthreads();
   // the next colour's CTAs may be scheduled as this grid's CTAs retire
-  if (p.pdl) grid_dep_launch_dependents();
+  if (LOCAL || p.pdl) grid_dep_launch_dependents();
   // launched as a dependent of the previous colour: dst is read only after
   // grid_dep_wait, which the first group of each warp does after its compute
-  bool dep_pending = p.pdl != 0;
+  bool dep_pending = !LOCAL && p.pdl != 0;
 
   unsigned char *base = smem_raw + ((kSmemAlign - (smem_u32(smem_raw) & (kSmemAlign - 1))) & (kSmemAlign - 1));
   Real *wsm = reinterpret_cast<Real *>(base) + warp * warp_smem_elems<P, Real, GEOM, GROUP>(NEWT ? 2 : gvel ? 1 : 0);
@@ -429,23 +491,40 @@ __global__ void __launch_bounds__(kWarpsPerCTA * 32, WOcc<P, Real>::min_blocks)
   Real *t1 = tiles + L::t0_elems + s_sub * L::sc1;
   // DoF offsets are 32-bit: the launcher checks that the lattice has < 2^32 DoFs
   const unsigned NXu = (unsigned)p.NX, NYu = (unsigned)p.NY, zs = NXu * NYu;
-  const int count = (int)p.ccount;
+  const int count = LOCAL ? runs.groups[8] * CPW : (int)p.ccount;  // LOCAL: groups of all colours
   const int gstride = gridDim.x * GPC;
   unsigned phase = 0;
 
+  // the run of group grp: its colour, the colour-local index of the group's first
+  // cell, the colour's cells and its first cell in colour-major order
+  struct Run {
+    int c, c0, cells;
+    long first;
+  };
+  auto run_of = [&](int grp) -> Run {
+    if constexpr (LOCAL) {
+      int c = 0;
+#pragma unroll
+      for (int e = 1; e < 8; ++e) c += grp >= runs.groups[e];
+      return Run{c, (grp - runs.groups[c]) * CPW, runs.count[c], runs.first[c]};
+    } else {
+      return Run{0, grp * CPW, count, p.cfirst};
+    }
+  };
   auto issue_stage = [&](int grp) {
-    const int c0 = grp * CPW;
-    const int ncell = min(CPW, count - c0);
+    const Run rn = run_of(grp);
+    const int c0 = rn.c0;
+    const int ncell = min(CPW, rn.cells - c0);
     const unsigned mb = ncell * MS * sizeof(Real), vb = gvel ? ncell * VS * sizeof(Real) : 0;
     fence_proxy_async();
     mbar_expect_tx(&bars[warp], mb + vb);
     if (p.stream_evict_first) {
       const uint64_t pol = l2_policy_evict_first();
-      bulk_g2s_hint(stage, p.metric + (p.cfirst + c0) * (long)MS, mb, &bars[warp], pol);
-      if (gvel) bulk_g2s_hint(vstage, p.velb + (p.cfirst + c0) * (long)VS, vb, &bars[warp], pol);
+      bulk_g2s_hint(stage, p.metric + (rn.first + c0) * (long)MS, mb, &bars[warp], pol);
+      if (gvel) bulk_g2s_hint(vstage, p.velb + (rn.first + c0) * (long)VS, vb, &bars[warp], pol);
     } else {
-      bulk_g2s(stage, p.metric + (p.cfirst + c0) * (long)MS, mb, &bars[warp]);
-      if (gvel) bulk_g2s(vstage, p.velb + (p.cfirst + c0) * (long)VS, vb, &bars[warp]);
+      bulk_g2s(stage, p.metric + (rn.first + c0) * (long)MS, mb, &bars[warp]);
+      if (gvel) bulk_g2s(vstage, p.velb + (rn.first + c0) * (long)VS, vb, &bars[warp]);
     }
   };
   // raw src column and constrained-DoF mask of the lane's cell in group grp;
@@ -459,10 +538,16 @@ __global__ void __launch_bounds__(kWarpsPerCTA * 32, WOcc<P, Real>::min_blocks)
   // store needs a lane predicate (only the global scatter is restricted to
   // lane_ok lanes)
   auto gather = [&](int grp, Real (&A)[n], uint4 &cm, int &ix, int &iy, int &iz, unsigned &g0) {
-    const int cidx = grp * CPW + sub;
-    const bool act = grp * CPW < count && cidx < count;
+    const bool in = grp * CPW < count;
+    const Run rn = run_of(in ? grp : 0);
+    const int cidx = rn.c0 + sub;
+    const bool act = in && cidx < rn.cells;
     ix = 0, iy = 0, iz = 0;
-    if (act) colour_cell(cidx, p, ix, iy, iz);
+    if constexpr (LOCAL) {
+      if (act) runs.cell(rn.c, cidx, ix, iy, iz);
+    } else {
+      if (act) colour_cell(cidx, p, ix, iy, iz);
+    }
     g0 = ((unsigned)(iz * P) * NYu + (unsigned)(iy * P + j)) * NXu + (unsigned)(ix * P + i);
     if (HANG && act && ix == 0 && i == 0) {
       // hanging DoF (0, j, k): the coarse face's interpolant at the fine node,
@@ -495,7 +580,7 @@ __global__ void __launch_bounds__(kWarpsPerCTA * 32, WOcc<P, Real>::min_blocks)
 #pragma unroll
       for (int k = 0; k < n; ++k) A[k] = act ? p.src[g0 + k * zs] : Real(0);
     }
-    cm = (act && use_mask) ? p.cell_mask[p.cfirst + cidx] : make_uint4(0u, 0u, 0u, 0u);
+    cm = (act && use_mask) ? p.cell_mask[rn.first + cidx] : make_uint4(0u, 0u, 0u, 0u);
   };
   auto mask_bit = [&](const uint4 &cm, int k) -> bool {
     const int b = k * n2 + l;
@@ -514,8 +599,9 @@ __global__ void __launch_bounds__(kWarpsPerCTA * 32, WOcc<P, Real>::min_blocks)
   for (; group * CPW < count; group += gstride) {
     const int gnext = group + gstride;
     const bool has_next = gnext * CPW < count;
-    const int cidx = group * CPW + sub;
-    const bool active = lane_ok && cidx < count;
+    const Run rn = run_of(group);
+    const int cidx = rn.c0 + sub;
+    const bool active = lane_ok && cidx < rn.cells;
     const int ix = nix, iy = niy, iz = niz;
     const unsigned g0 = ng0;
     // constrained DoFs of the lane's column (bit k: DoF (i, j, k)); skipped as a
@@ -566,7 +652,7 @@ __global__ void __launch_bounds__(kWarpsPerCTA * 32, WOcc<P, Real>::min_blocks)
 #pragma unroll
       for (int k = 0; k < n; ++k) {
         const bool first = (first_bits >> k) & 1, masked = (mask_bits >> k) & 1;
-        dpre[k] = (active && !first && !masked && !hl) ? dst_v[gk[k]] : Real(0);
+        dpre[k] = (!LOCAL && active && !first && !masked && !hl) ? dst_v[gk[k]] : Real(0);
       }
     };
     if (!late_dst) load_dpre();
@@ -579,7 +665,7 @@ __global__ void __launch_bounds__(kWarpsPerCTA * 32, WOcc<P, Real>::min_blocks)
     } else {
       const Real *src_v = p.msrc[v];
 #pragma unroll
-      for (int k = 0; k < n; ++k) u[k] = (cidx < count) ? src_v[g0 + k * zs] : Real(0);
+      for (int k = 0; k < n; ++k) u[k] = (cidx < rn.cells) ? src_v[g0 + k * zs] : Real(0);
     }
     if (any_mask) {
 #pragma unroll
@@ -601,7 +687,7 @@ __global__ void __launch_bounds__(kWarpsPerCTA * 32, WOcc<P, Real>::min_blocks)
       uniform_velocity<Real, n>(p, T, ix, iy, iz, i, j, 0, uv0);
     // velocity given as a DoF vector on a uniform mesh: the stream JxW J^-1 u,
     // read from global memory (lanes of a cell read consecutive values)
-    const Real *vq = nodal_vel ? p.velb + (p.cfirst + (cidx < count ? cidx : 0)) * (long)VS + j * n + i : nullptr;
+    const Real *vq = nodal_vel ? p.velb + (rn.first + (cidx < rn.cells ? cidx : 0)) * (long)VS + j * n + i : nullptr;
 
     Real val[n], fx[n], fy[n], fz[n];
     const Real *ms = stage + s_sub * MS + j * n + i;
@@ -693,7 +779,13 @@ __global__ void __launch_bounds__(kWarpsPerCTA * 32, WOcc<P, Real>::min_blocks)
       load_dpre();
     }
 
-    if (!HANG && !any_mask) {
+    if constexpr (LOCAL) {
+      if (active) {
+        Real *o = p.local + (rn.first + cidx) * (long)n3 + l;
+#pragma unroll
+        for (int k = 0; k < n; ++k) o[k * n2] = out[k];
+      }
+    } else if (!HANG && !any_mask) {
       // no constrained DoF in the warp's cells: dpre is 0 where the cell stores first
       if (active) {
 #pragma unroll

@@ -217,6 +217,10 @@ struct Op {
   double *d_flux64 = nullptr;
   float *d_flux32 = nullptr;
   bool fields_frozen = false;  // inside a linear solve: the fields do not change
+  // small lattices: the cells' results of one apply, before they are gathered
+  void *d_local = nullptr;
+  size_t local_bytes = 0;
+  bool no_build = false;       // inside a solve that may not allocate
   size_t device_bytes = 0;
   // two-level mesh: the fine block's operator and the per-interface-cell stage
   // of the hanging DoFs' contributions to the coarse DoFs

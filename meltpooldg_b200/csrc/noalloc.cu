@@ -82,6 +82,11 @@ int solve_cg_noalloc(Op &op, double *x, const double *b, double rel_tol, double 
   if (N > kNoAllocMaxDofs)
     throw Error{MPDG_ERR_SIZE, "problem has " + std::to_string(N) + " DoFs; the allocation-free CG "
                 "holds scratch for at most " + std::to_string(kNoAllocMaxDofs)};
+  struct NoBuild {
+    Op &op;
+    ~NoBuild() { op.no_build = false; }
+  } no_build{op};
+  op.no_build = true;
   if (const char *why = noalloc_unready_reason(op))
     throw Error{MPDG_ERR_ARG, std::string("mpdg_solve_cg_noalloc: ") + why};
   double *base = scratch_for_current_device();

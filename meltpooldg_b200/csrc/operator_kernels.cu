@@ -265,6 +265,7 @@ struct KP {
   const uint8_t *dmask;
   const uint8_t *cell_flags;
   const uint4 *cell_mask;
+  Real *local;            // LOCAL apply: the cells' results [colour-major cell][n^3]
   const uint4 *cell_first;  // mapped meshes: first-touch local DoFs per cell (null: every cell adds)
   long NX, NY;
   int nc[3];
@@ -1684,22 +1685,26 @@ void build_mesh_device_data(Mesh &m, const uint8_t *host_mask, bool force_genera
         const int iz = 2 * (int)(k / ((long)C.cn[0] * C.cn[1])) + C.par[2];
         uint8_t f = 0;
         for (int kk = 0; kk <= p; ++kk)
-          for (int jj = 0; jj <= p; ++jj)
+          for (int jj = 0; jj <= p; ++jj) {
+            const uint8_t *row = host_mask + ((long)(iz * p + kk) * m.NY + (iy * p + jj)) * m.NX + ix * p;
+            unsigned any_in_row = 0;
+            for (int ii = 0; ii <= p; ++ii) any_in_row |= row[ii];
+            if (!any_in_row) continue;
             for (int ii = 0; ii <= p; ++ii) {
-              const long g = ((long)(iz * p + kk) * m.NY + (iy * p + jj)) * m.NX + (ix * p + ii);
-              if (host_mask[g]) {
+              if (row[ii]) {
                 f = 1;
                 const int bit = (kk * n + jj) * n + ii;
                 cmask[4 * (C.first + k) + bit / 32] |= 1u << (bit % 32);
               }
             }
+          }
         flags[C.first + k] = f;
         any = any || f;
       }
     }
     m.has_dirichlet = any;
-    // a mask that is a union of whole box faces (bit 2 d + side)
-    if (any) {
+    // a mask that is a union of whole box faces (bit 2 d + side), for the band apply
+    if (any && uniform) {
       const long NXY = m.NX * m.NY;
       auto face_of = [&](int f, long a, long b) {  // DoF (a, b) of face f
         const int d = f / 2;
@@ -2144,6 +2149,80 @@ int num_sms()
   return g_num_sms;
 }
 
+// Small lattices apply in two launches -- all cells into local results, then a
+// gather per DoF -- instead of eight colours, whose launches take 23 us whatever the
+// size; the extra pass over n^3 values per cell stays in the L2.  Measured (general
+// cells, FP64 / FP32, us, coloured -> this): 8^3 Q2 24 -> 8.3 / 23 -> 7.8, 20^3 Q3
+// 26 -> 16.5 / 27 -> 14.4, 16^3 Q4 24 -> 19.8 / 23 -> 15.3, 40x32x24 Q2 (829k values)
+// 24 -> 24.8 / 24 -> 18.5; 25^3 Q4 (1.95M values) 46 -> 49 / 30 -> 37: hence the line.
+// The sums are the coloured apply's, bit for bit.
+constexpr long kLocalValues = 900000;  // n_cells n^3 at most
+template <typename Real>
+bool local_apply_fits(const Op &op, const KP<Real> &k)
+{
+  const Mesh &m = *op.mesh;
+  if (m.mapped || k.hsrc || k.nvec > 1 || k.zhi > k.zlo || m.NY > 65535 || m.NZ > 65535) return false;
+  const size_t bytes = sizeof(Real) * (size_t)m.n_cells * m.n * m.n * m.n;
+  return m.n_cells * m.n * m.n * m.n <= kLocalValues && (op.local_bytes >= bytes || !op.no_build);
+}
+
+template <int P, typename Real, int GEOM, bool NEWT = false>
+void run_local_apply(Op &op, KP<Real> k)
+{
+  Mesh &m = *op.mesh;
+  constexpr int n = P + 1, CPW = 32 / (n * n);
+  const bool gvel = GEOM == GEOM_GENERAL && (NEWT || op.d.vel_kind != MPDG_VEL_NONE);
+  const size_t smem = sizeof(Real) * warp_smem_elems<P, Real, GEOM>(NEWT ? 2 : gvel ? 1 : 0) * kWarpsPerCTA + kSmemAlign;
+  if (GEOM == GEOM_GENERAL && (!k.metric || (gvel && !k.velb))) throw Error{MPDG_ERR_ARG, "coefficient stream missing"};
+  const size_t bytes = sizeof(Real) * (size_t)m.n_cells * n * n * n;
+  if (op.local_bytes < bytes) {
+    MPDG_CUDA(cudaStreamSynchronize(op.stream));
+    if (op.d_local) cudaFree(op.d_local);
+    op.d_local = nullptr;
+    op.local_bytes = 0;
+    MPDG_CUDA(tracked_malloc(&op.d_local, bytes));
+    op.local_bytes = bytes;
+  }
+  k.local = static_cast<Real *>(op.d_local);
+  auto kern = warp_apply_kernel<P, Real, GEOM, false, false, false, 32, NEWT, true>;
+  static int configured_smem = -1, blocks_per_sm = 0;  // per instantiation
+  if (configured_smem != (int)smem) {
+    MPDG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    MPDG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, kern, kWarpsPerCTA * 32, smem));
+    if (blocks_per_sm < 1) blocks_per_sm = 1;
+    configured_smem = (int)smem;
+  }
+  ColourRuns runs{};
+  for (int c = 0; c < 8; ++c) {
+    const Colour &C = m.colour[c];
+    colour_params(k, C);  // checks the index arithmetic
+    runs.count[c] = (int)C.count;
+    runs.first[c] = C.first;
+    runs.cn0[c] = C.cn[0];
+    runs.cn1[c] = C.cn[1];
+    runs.m0[c] = k.div0_magic;
+    runs.m01[c] = k.div01_magic;
+    runs.groups[c + 1] = runs.groups[c] + (int)((C.count + CPW - 1) / CPW);
+  }
+  k.stream_evict_first = 0;
+  k.pdl = 0;
+  const long blocks = std::min((long)num_sms() * blocks_per_sm, (long)(runs.groups[8] + kWarpsPerCTA - 1) / kWarpsPerCTA);
+  kern<<<(unsigned)blocks, kWarpsPerCTA * 32, smem, op.stream>>>(k, op.d_err, runs);
+  MPDG_LAUNCHED();
+  // the gather starts as the cells' CTAs retire and waits before its first read
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)((m.NX + 127) / 128), (unsigned)m.NY, (unsigned)m.NZ);
+  cfg.blockDim = dim3(128);
+  cfg.stream = op.stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  MPDG_CUDA(cudaLaunchKernelEx(&cfg, local_gather_kernel<P, Real>, k, runs));
+  MPDG_LAUNCHED();
+}
+
 template <int P, typename Real, int GEOM, bool HANG, bool MULTI = false, bool MAPPED = false, int GROUP = 32,
           bool NEWT = false>
 void run_warp_apply(Op &op, KP<Real> k)
@@ -2211,7 +2290,7 @@ void run_warp_apply(Op &op, KP<Real> k)
       attr[0].val.programmaticStreamSerializationAllowed = 1;
       cfg.attrs = attr;
       cfg.numAttrs = pdl ? 1 : 0;
-      MPDG_CUDA(cudaLaunchKernelEx(&cfg, kern, k, op.d_err));
+      MPDG_CUDA(cudaLaunchKernelEx(&cfg, kern, k, op.d_err, ColourRuns{}));
       MPDG_LAUNCHED();
       ++launched;
     }
@@ -2464,6 +2543,16 @@ void warp_apply_degree(Op &op, const KP<Real> &k)
       return;
     }
   }
+  if (local_apply_fits(op, k)) {
+    switch (op.mesh->degree) {
+      case 1: run_local_apply<1, Real, GEOM>(op, k); break;
+      case 2: run_local_apply<2, Real, GEOM>(op, k); break;
+      case 3: run_local_apply<3, Real, GEOM>(op, k); break;
+      case 4: run_local_apply<4, Real, GEOM>(op, k); break;
+      default: throw Error{MPDG_ERR_UNSUPPORTED, "degree must be 1..4"};
+    }
+    return;
+  }
   if (k.nvec > 1) {
     switch (op.mesh->degree) {
       case 1: run_warp_apply<1, Real, GEOM, false, true>(op, k); break;
@@ -2610,8 +2699,14 @@ void frozen_field_apply(Op &op, KP<Real> k)
   k.c_vel = Real(1);
   auto run = [&](auto deg) {
     constexpr int P = decltype(deg)::value;
-    if (flux) run_warp_apply<P, Real, GEOM_GENERAL, false, false, false, 32, true>(op, k);
-    else run_warp_apply<P, Real, GEOM_GENERAL, false>(op, k);
+    if (local_apply_fits(op, k)) {
+      if (flux) run_local_apply<P, Real, GEOM_GENERAL, true>(op, k);
+      else run_local_apply<P, Real, GEOM_GENERAL>(op, k);
+    } else if (flux) {
+      run_warp_apply<P, Real, GEOM_GENERAL, false, false, false, 32, true>(op, k);
+    } else {
+      run_warp_apply<P, Real, GEOM_GENERAL, false>(op, k);
+    }
   };
   switch (op.mesh->degree) {
     case 1: run(std::integral_constant<int, 1>{}); break;
