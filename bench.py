@@ -60,12 +60,10 @@ WL = {"name": "heat", "nc": [64, 64, 64], "degree": 4}
 # the cells of a 64^3 apply (262,144 / 110,592), as traffic grows with the
 # cells processed; the level-set workload's capture is at full size
 # (profiles/warp_apply_q2_uniform_128c.md: 381.4 MB over two launches).  The
-# lane apply (one thread per Q2 cell, the level-set workload's default) was
-# captured at full size over all 8 colour launches of an apply with the cache
-# left warm between launches (profiles/lane_apply_q2_uniform_128c.md: 481.8 MB
-# read, 298.4 MB written).
+# band apply (the level-set workload's default) was captured at full size in its one
+# launch (profiles/band_apply_q2_uniform_128c.md).
 MEASURED_TRAFFIC_BYTES = {("heat", 64, "warp"): 2.720e9, ("advdiff", 128, "warp"): 1.526e9,
-                         ("advdiff", 128, "lane"): 0.780e9}
+                         ("advdiff", 128, "band"): 0.232e9}
 
 
 def set_workload(name, cells=0):
@@ -118,7 +116,7 @@ def apply_kernel_name(op, p, geom):
     """The FP64 apply kernel the operator's schedule runs."""
     sc = op.schedule("fp64")
     if sc["lane_cells"] and geom == "UNIFORM" and p <= 2:
-        return f"lane_apply_kernel<{p},double> x {4 if WL['nc'][0] <= 32 else 8} colour launches"
+        return f"band_apply_kernel<{p},double> x 1 launch"
     return f"warp_apply_kernel<{p},double,{geom}> x 8 colour launches"
 
 
@@ -493,7 +491,7 @@ def run_operator_workload(args, rank, world, headline):
     geom = "UNIFORM" if WL["name"] in ("advdiff", "c1") else "GENERAL"
     b64, b32 = algorithmic_bytes(N, E, p, 8), algorithmic_bytes(N, E, p, 4)
     st64, st32 = streamed_bytes(N, E, p, 8), streamed_bytes(N, E, p, 4)
-    kernel_kind = "lane" if apply_kernel_name(op, p, geom).startswith("lane") else "warp"
+    kernel_kind = "band" if apply_kernel_name(op, p, geom).startswith("band") else "warp"
     traffic = MEASURED_TRAFFIC_BYTES.get((WL["name"], nc[0], kernel_kind))
     roof = {"bound": "hbm", "achieved": b64 / apply_s / 1e9, "peak": peak, "unit": "GB/s",
             "frac": b64 / apply_s / 1e9 / peak, "traffic": traffic,

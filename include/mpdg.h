@@ -291,12 +291,13 @@ mpdg_status mpdg_vmult_multi(mpdg_op *op, int n_vectors, double *const *dst, con
  * cells (5 Q4 cells or 14 Q2 cells per 128 threads instead of 4 or 12, so
  * fewer lanes idle; the tile exchanges become CTA barriers), for degrees 2
  * and 4 on lattice meshes.  lane_cells (uniform lattices of degree 1 or 2,
- * constant coefficients, one operand, velocities other than MPDG_VEL_NODAL)
- * gives every cell one thread that keeps its whole sum factorisation in
- * registers; 32 lanes own a row segment of cells and add their shared x-faces
- * by warp shuffles, so these launches colour by segment parity in x.  Results
- * are identical for every schedule without lane_cells, and agree with them to
- * rounding with it.  No reference
+ * constant coefficients, velocities other than MPDG_VEL_NODAL) selects the band
+ * apply, which applies the operator as sums of products of line matrices; it is
+ * the default there, and on uniform lattices of degree 3 and 4 until a schedule is
+ * set.  Results are identical for every schedule without lane_cells, and agree
+ * with them to rounding with it; lattices of at most 900,000 local values (cells
+ * times (degree + 1)^3) run in two launches whatever the schedule says, with the
+ * same bits.  No reference
  * counterpart: the schedule of deal.II's MatrixFree::cell_loop
  * (heat_diffuse_operator.cpp:183) is internal to it. */
 typedef struct {
@@ -304,14 +305,14 @@ typedef struct {
   int l2_evict_first;   /* 0 or 1 */
   int overlap_colours;  /* 0 or 1 */
   int cta_cell_groups;  /* 0 or 1 */
-  int lane_cells;       /* 0: warp apply; 1, 2: lane apply, 2 with more resident CTAs per SM */
+  int lane_cells;       /* 0: warp apply; 1, 2: band apply */
 } mpdg_schedule;
 mpdg_status mpdg_op_set_schedule(mpdg_op *op, int precision, const mpdg_schedule *schedule);
 mpdg_status mpdg_op_get_schedule(mpdg_op *op, int precision, mpdg_schedule *schedule);
 /* Autotuner of the resident apply: times `reps` applies (after one warm-up) of
- * each candidate schedule -- slabs 1, 2, 4, 8, 16, each with and without the
- * evict-first hint where the mesh streams coefficients, each with and without
- * overlap_colours -- in the given
+ * each candidate schedule -- the operator's own first, then slabs 1 and 2, each with
+ * and without the evict-first hint where the mesh streams coefficients, each with
+ * and without overlap_colours, cta_cell_groups and lane_cells where they apply -- in the given
  * precision (MPDG_FP64 / MPDG_FP32), keeps the fastest on the operator and
  * returns it with its time per apply.  candidate_ms (may be NULL) receives up to
  * n_candidate_ms per-candidate times in that order (-1 past the last).

@@ -257,9 +257,9 @@ mpdg_status mpdg_op_create(mpdg_mesh *mesh, const mpdg_op_desc *desc, mpdg_op **
     // 64^3 Q4 FP64 0.490 -> 0.485 ms; Q4 FP32 0.294 -> 0.299 ms, kept on warps)
     o.sched[MPDG_FP64].cta = (mm.degree == 2 || mm.degree == 4) ? 1 : 0;
     o.sched[MPDG_FP32].cta = mm.degree == 2 ? 1 : 0;
-    // what the schedule reports where the band apply serves Q1/Q2; it runs by
-    // default on every lattice it serves, whatever the size and degree
-    const int lane_default = (mm.degree == 2 && mm.n_cells >= 32768) ? 1 : 0;
+    // the band apply serves uniform lattices of degree 1 and 2 by default; the
+    // schedule reports it as lane_cells (degrees 3 and 4: not a schedule option)
+    const int lane_default = mm.degree <= 2 ? 1 : 0;
     o.sched[MPDG_FP64].lane = lane_default;
     o.sched[MPDG_FP32].lane = lane_default;
     try {

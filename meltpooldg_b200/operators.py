@@ -266,9 +266,10 @@ class _MatrixFreeOperator:
         slab by slab over `slabs` z-slabs of cell layers, the L2 evict-first
         hint on the coefficient stream, colour launches that overlap the
         previous colour's tail (programmatic dependent launch), cell groups
-        shared by a whole CTA (degrees 2 and 4), and one thread per cell
-        (lane_cells 1 or 2: uniform lattices of degree 1 or 2).  Results do not
-        depend on it, except for rounding with lane_cells."""
+        shared by a whole CTA (degrees 2 and 4), and the band apply
+        (lane_cells 1 or 2: uniform lattices of degree 1 or 2, the default
+        there).  Results do not depend on it, except for rounding with
+        lane_cells."""
         s = A.Schedule(int(slabs), int(bool(l2_evict_first)), int(bool(overlap_colours)), int(bool(cta_cell_groups)),
                        int(lane_cells))
         A.check(A.lib().mpdg_op_set_schedule(self._h, A.FP32 if precision == "fp32" else A.FP64, C.byref(s)),
