@@ -292,7 +292,9 @@ namespace {
 void free_op_arrays(Op &o)
 {
   free_workspace(o);
-  for (void *p : {(void *)o.T_own, (void *)o.d_err, (void *)o.d_coef64, (void *)o.d_coef32, (void *)o.d_flux64, (void *)o.d_flux32, o.d_local, (void *)o.T32, (void *)o.Ts32,
+  for (void *p : o.d_local)
+    if (p) cudaFree(p);
+  for (void *p : {(void *)o.T_own, (void *)o.d_err, (void *)o.d_coef64, (void *)o.d_coef32, (void *)o.d_flux64, (void *)o.d_flux32, (void *)o.T32, (void *)o.Ts32,
                   (void *)o.d_velb64, (void *)o.d_velb32, (void *)o.d_trig32, (void *)o.d_trig64, o.d_stage,
                   (void *)o.d_tau64, (void *)o.d_tau32, (void *)o.d_lam64, (void *)o.d_lam32, (void *)o.Told_own, (void *)o.H_own, (void *)o.Told32,
                   (void *)o.H32, (void *)o.lsq_buf, (void *)o.host_stage,
@@ -447,7 +449,15 @@ mpdg_status mpdg_op_set_inflow_outflow(mpdg_op *op, const uint8_t *host_mask)
 mpdg_status mpdg_op_set_stream(mpdg_op *op, void *stream)
 {
   if (!op) return MPDG_ERR_ARG;
-  op->o.stream = (cudaStream_t)stream;
+  Op &o = op->o;
+  o.stream = (cudaStream_t)stream;
+  o.local_slot = -1;
+  for (int i = 0; i < o.local_streams; ++i)
+    if (o.local_stream[i] == o.stream) o.local_slot = i;
+  if (o.local_slot < 0 && o.local_streams < Op::kLocalStreams) {
+    o.local_slot = o.local_streams++;
+    o.local_stream[o.local_slot] = o.stream;
+  }
   if (op->o.fine) op->o.fine->stream = (cudaStream_t)stream;
   return MPDG_OK;
 }

@@ -217,9 +217,16 @@ struct Op {
   double *d_flux64 = nullptr;
   float *d_flux32 = nullptr;
   bool fields_frozen = false;  // inside a linear solve: the fields do not change
-  // small lattices: the cells' results of one apply, before they are gathered
-  void *d_local = nullptr;
-  size_t local_bytes = 0;
+  bool merge_declined = false;  // that solve's streams would take too much of the free memory
+  // small lattices: the cells' results of one apply, before they are gathered; one
+  // buffer per stream that the operator was set to (a further stream has none and
+  // takes the coloured launches, which need no workspace), FP64-sized, kept in
+  // place until the operator goes
+  static constexpr int kLocalStreams = 4;
+  void *d_local[kLocalStreams] = {};
+  cudaStream_t local_stream[kLocalStreams] = {};
+  int local_streams = 1;       // slots given out; slot 0 is the default stream's
+  int local_slot = 0;          // of the stream set last; -1: none left
   bool no_build = false;       // inside a solve that may not allocate
   size_t device_bytes = 0;
   // two-level mesh: the fine block's operator and the per-interface-cell stage

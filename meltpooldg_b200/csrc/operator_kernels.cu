@@ -2157,13 +2157,30 @@ int num_sms()
 // 24 -> 24.8 / 24 -> 18.5; 25^3 Q4 (1.95M values) 46 -> 49 / 30 -> 37: hence the line.
 // The sums are the coloured apply's, bit for bit.
 constexpr long kLocalValues = 900000;  // n_cells n^3 at most
+// Under a caller's capture the coloured launches stay: a graph may be replayed on any
+// stream, beside applies that use the same workspace (a solve's own capture, made with
+// fields_frozen, runs on the solve's stream).
 template <typename Real>
-bool local_apply_fits(const Op &op, const KP<Real> &k)
+bool local_apply_ready(Op &op, const KP<Real> &k)
 {
   const Mesh &m = *op.mesh;
   if (m.mapped || k.hsrc || k.nvec > 1 || k.zhi > k.zlo || m.NY > 65535 || m.NZ > 65535) return false;
-  const size_t bytes = sizeof(Real) * (size_t)m.n_cells * m.n * m.n * m.n;
-  return m.n_cells * m.n * m.n * m.n <= kLocalValues && (op.local_bytes >= bytes || !op.no_build);
+  const long values = m.n_cells * m.n * m.n * m.n;
+  if (values > kLocalValues || op.local_slot < 0) return false;
+  if (!op.fields_frozen) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(op.stream, &st) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    if (st != cudaStreamCaptureStatusNone) return false;
+  }
+  void *&buf = op.d_local[op.local_slot];
+  if (!buf && !op.no_build && tracked_malloc(&buf, sizeof(double) * (size_t)values) != cudaSuccess) {
+    cudaGetLastError();
+    buf = nullptr;
+  }
+  return buf != nullptr;
 }
 
 template <int P, typename Real, int GEOM, bool NEWT = false>
@@ -2174,16 +2191,7 @@ void run_local_apply(Op &op, KP<Real> k)
   const bool gvel = GEOM == GEOM_GENERAL && (NEWT || op.d.vel_kind != MPDG_VEL_NONE);
   const size_t smem = sizeof(Real) * warp_smem_elems<P, Real, GEOM>(NEWT ? 2 : gvel ? 1 : 0) * kWarpsPerCTA + kSmemAlign;
   if (GEOM == GEOM_GENERAL && (!k.metric || (gvel && !k.velb))) throw Error{MPDG_ERR_ARG, "coefficient stream missing"};
-  const size_t bytes = sizeof(Real) * (size_t)m.n_cells * n * n * n;
-  if (op.local_bytes < bytes) {
-    MPDG_CUDA(cudaStreamSynchronize(op.stream));
-    if (op.d_local) cudaFree(op.d_local);
-    op.d_local = nullptr;
-    op.local_bytes = 0;
-    MPDG_CUDA(tracked_malloc(&op.d_local, bytes));
-    op.local_bytes = bytes;
-  }
-  k.local = static_cast<Real *>(op.d_local);
+  k.local = static_cast<Real *>(op.d_local[op.local_slot]);
   auto kern = warp_apply_kernel<P, Real, GEOM, false, false, false, 32, NEWT, true>;
   static int configured_smem = -1, blocks_per_sm = 0;  // per instantiation
   if (configured_smem != (int)smem) {
@@ -2452,7 +2460,8 @@ void run_band(Op &op, const KP<Real> &k, bool add)
     const long tiles = (long)b.ntx * b.nty;
     const int nz = zhi - zlo;
     long best = -1;
-    for (int len = 1; len <= nz; ++len) {
+    for (int want = std::min(nz, 4096); want >= 1; --want) {  // the shortest chunks of each number of chunks
+      const int len = (nz + want - 1) / want;
       const long chunks = (nz + len - 1) / len;
       const long cost = ((tiles * chunks + resident - 1) / resident) * (len + (chunks > 1 || zlo > 0 ? 1 : 0));
       if (best < 0 || cost <= best) {
@@ -2543,7 +2552,7 @@ void warp_apply_degree(Op &op, const KP<Real> &k)
       return;
     }
   }
-  if (local_apply_fits(op, k)) {
+  if (local_apply_ready(op, k)) {
     switch (op.mesh->degree) {
       case 1: run_local_apply<1, Real, GEOM>(op, k); break;
       case 2: run_local_apply<2, Real, GEOM>(op, k); break;
@@ -2638,14 +2647,22 @@ bool live_fields(const Op &op)
 // whether such an operator has velocity or Newton flux values beside the coefficients
 bool field_fluxes(const Op &op) { return uses_law(op) || op.d.full_tangent || op.d.vel_kind != MPDG_VEL_NONE; }
 
+// False where the streams would take more than a quarter of the free device memory
+// (the solver's vectors come after them): the solve then evaluates the fields in
+// every apply, which needs no memory per cell.
 template <typename Real>
-void ensure_field_coef(Op &op)
+bool ensure_field_coef(Op &op)
 {
   Mesh &m = *op.mesh;
   constexpr bool f32 = sizeof(Real) == 4;
   bool &ok = f32 ? op.coef32_ok : op.coef64_ok;
-  if (ok) return;
+  if (ok) return true;
   const size_t count = (size_t)m.n_cells * metric_stride(m.n), fcount = 2 * (size_t)m.n_cells * velb_stride(m.n);
+  if (f32 ? !op.d_coef32 : !op.d_coef64) {
+    size_t free_bytes = 0, total = 0;
+    MPDG_CUDA(cudaMemGetInfo(&free_bytes, &total));
+    if (sizeof(Real) * (count + (field_fluxes(op) ? fcount : 0)) > free_bytes / 4) return false;
+  }
   auto buffer = [&](auto *&p, size_t cnt) {  // padding is copied, never read
     using R = std::remove_reference_t<decltype(*p)>;
     if (p) return;
@@ -2682,12 +2699,17 @@ void ensure_field_coef(Op &op)
     default: throw Error{MPDG_ERR_UNSUPPORTED, "degree must be 1..4"};
   }
   ok = true;
+  return true;
 }
 
 template <typename Real>
-void frozen_field_apply(Op &op, KP<Real> k)
+bool frozen_field_apply(Op &op, KP<Real> k)
 {
-  ensure_field_coef<Real>(op);
+  if (op.merge_declined || op.mesh->N >= (1L << 32)) return false;  // (the warp apply's 32-bit offsets)
+  if (!ensure_field_coef<Real>(op)) {
+    op.merge_declined = true;
+    return false;
+  }
   const bool flux = field_fluxes(op);
   if constexpr (sizeof(Real) == 8) {
     k.metric = op.d_coef64;
@@ -2699,7 +2721,7 @@ void frozen_field_apply(Op &op, KP<Real> k)
   k.c_vel = Real(1);
   auto run = [&](auto deg) {
     constexpr int P = decltype(deg)::value;
-    if (local_apply_fits(op, k)) {
+    if (local_apply_ready(op, k)) {
       if (flux) run_local_apply<P, Real, GEOM_GENERAL, true>(op, k);
       else run_local_apply<P, Real, GEOM_GENERAL>(op, k);
     } else if (flux) {
@@ -2715,6 +2737,7 @@ void frozen_field_apply(Op &op, KP<Real> k)
     case 4: run(std::integral_constant<int, 4>{}); break;
     default: throw Error{MPDG_ERR_UNSUPPORTED, "degree must be 1..4"};
   }
+  return true;
 }
 
 }  // namespace
@@ -2972,6 +2995,7 @@ void launch_robin(Op &op, Real *dst, const Real *src, int mode)
 FrozenFields::FrozenFields(Op &o) : op(o), was(o.fields_frozen)
 {
   if (!was && live_fields(op)) op.coef64_ok = op.coef32_ok = false;
+  if (!was) op.merge_declined = false;
   op.fields_frozen = true;
 }
 
@@ -3157,10 +3181,7 @@ void launch_cells(Op &op, Real *dst, const Real *src)
     return;
   }
   const bool law = uses_law(op);
-  if (op.fields_frozen && live_fields(op)) {
-    frozen_field_apply<Real>(op, k);
-    return;
-  }
+  if (op.fields_frozen && live_fields(op) && frozen_field_apply<Real>(op, k)) return;
   if (!full && !law && !m.uniform) {
     // general geometry: merged coefficient stream (k(T), c_mass, c_diff folded in)
     ensure_coef(op, sizeof(Real) == 4);

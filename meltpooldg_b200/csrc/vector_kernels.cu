@@ -42,13 +42,15 @@ __device__ __forceinline__ double block_sum(double v)
 }
 
 // True in the last block of the grid to get here: the blocks' partials written
-// before the call (by thread 0) are then visible to it.  The ticket counts the
+// before the call (by thread 0) are then visible to it, and all their threads have
+// read what they read before the call (the last block may overwrite the scalars).  The ticket counts the
 // blocks and is back at 0 afterwards; kernels of one stream may share it.  The last
 // block takes the place of a second launch that read the partials: at 36k DoFs a
 // CG iteration was 9 kernels of 2-4 us each and is 4 now.
 __device__ __forceinline__ bool last_block(double *ticket)
 {
   __shared__ bool last;
+  __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
     last = atomicInc(reinterpret_cast<unsigned *>(ticket), gridDim.x - 1) == gridDim.x - 1;
