@@ -421,6 +421,23 @@ __global__ void __launch_bounds__(128) local_gather_kernel(const KP<Real> p, con
   p.dst[g] = masked ? Real(0) : s;
 }
 
+// the same on a mapped mesh, through the inverse of the cell->DoF map; DoFs of no cell
+// get 0
+template <typename Real>
+__global__ void __launch_bounds__(128) mapped_gather_kernel(Real *dst, const Real *local, const int *ptr, const int *touch,
+                                                            const uint8_t *dmask, long N)
+{
+  const long g = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (g >= N) return;
+  const int b = ptr[g], e = ptr[g + 1];
+  const bool masked = dmask && dmask[g];
+  grid_dep_wait();
+  Real s = 0;
+#pragma unroll 4
+  for (int t = b; t < e; ++t) s += __ldcg(local + touch[t]);
+  dst[g] = masked ? Real(0) : s;
+}
+
 template <int P, typename Real>
 struct WOcc {
   static constexpr int min_blocks = (sizeof(Real) == 8) ? (P == 4 ? 3 : P == 3 ? 4 : P == 2 ? 5 : 6)
@@ -440,7 +457,8 @@ struct WOcc {
 // NEWT: the velocity stream holds, per cell, the scaled velocity values (c_vel = 1)
 // and then the Newton flux, which adds its values times u to the flux
 // LOCAL: all colours in one launch; a cell's results go to its n^3 values of p.local
-// (colour-major), which local_gather_kernel adds per DoF in colour order
+// (colour-major), which the gather kernels add per DoF in colour order (a mapped mesh's
+// cells are one run)
 template <int P, typename Real, int GEOM, bool HANG = false, bool MULTI = false, bool MAPPED = false,
           int GROUP = 32, bool NEWT = false, bool LOCAL = false>
 __global__ void __launch_bounds__(kWarpsPerCTA * 32, WOcc<P, Real>::min_blocks)
@@ -451,7 +469,7 @@ __global__ void __launch_bounds__(kWarpsPerCTA * 32, WOcc<P, Real>::min_blocks)
   static_assert(GROUP == 32 || (GROUP == kWarpsPerCTA * 32 && !HANG && !MULTI && !MAPPED),
                 "CTA-wide cell groups: plain applies only");
   static_assert(!NEWT || (GEOM == GEOM_GENERAL && GROUP == 32 && !HANG && !MULTI && !MAPPED), "Newton flux: plain general applies");
-  static_assert(!LOCAL || (GROUP == 32 && !HANG && !MULTI && !MAPPED), "local results: plain applies");
+  static_assert(!LOCAL || (GROUP == 32 && !HANG && !MULTI), "local results: plain applies");
   constexpr bool CTA = GROUP != 32;
   using L = TileLayout<P + 1, Real, GROUP>;
   constexpr int n = P + 1, n2 = n * n, n3 = n2 * n, CPW = GROUP / n2;
@@ -620,7 +638,7 @@ __global__ void __launch_bounds__(kWarpsPerCTA * 32, WOcc<P, Real>::min_blocks)
     unsigned gk[n];
 #pragma unroll
     for (int k = 0; k < n; ++k)
-      gk[k] = MAPPED ? (active ? (unsigned)p.cmap[(p.cfirst + cidx) * (long)n3 + k * n2 + l] : 0u) : g0 + k * zs;
+      gk[k] = MAPPED ? (!LOCAL && active ? (unsigned)p.cmap[(p.cfirst + cidx) * (long)n3 + k * n2 + l] : 0u) : g0 + k * zs;
 
     // hanging lane of the fine block: its column is the coarse face's interpolant,
     // its slots are never written (stored 0 by the first cell), its result is staged
@@ -634,7 +652,7 @@ __global__ void __launch_bounds__(kWarpsPerCTA * 32, WOcc<P, Real>::min_blocks)
     // cells) from the per-cell mask; none when the mesh has no masks (dst cleared)
     uint4 cfm = make_uint4(0u, 0u, 0u, 0u);
     if constexpr (MAPPED) {
-      if (p.cell_first && active) cfm = p.cell_first[p.cfirst + cidx];
+      if (!LOCAL && p.cell_first && active) cfm = p.cell_first[p.cfirst + cidx];
     }
 #pragma unroll
     for (int k = 0; k < n; ++k) {

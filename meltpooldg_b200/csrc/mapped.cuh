@@ -559,6 +559,15 @@ void build_mapped_mesh(Mesh &m, const mpdg_mapped_mesh_desc &d)
   size_t &B = m.device_bytes;
   m.d_cmap = upload(cmap, B);
   m.d_cell_first = upload(cfirst, B);
+  if (n_col > 2 && (long)cmap.size() <= mapped_local_values(p)) {
+    std::vector<int> ptr((size_t)N + 1, 0), touch(cmap.size());
+    for (const int g : cmap) ++ptr[g + 1];
+    for (long g = 0; g < N; ++g) ptr[g + 1] += ptr[g];
+    std::vector<int> at(ptr.begin(), ptr.end() - 1);
+    for (size_t e = 0; e < cmap.size(); ++e) touch[at[cmap[e]]++] = (int)e;
+    m.d_touch_ptr = upload(ptr, B);
+    m.d_touch = upload(touch, B);
+  }
   // boundary faces: greedy face colours (no two faces of a colour share a DoF)
   if (d.face_ids) {
     std::vector<uint64_t> fused(N, 0);

@@ -148,6 +148,9 @@ struct Mesh {
   bool mapped = false;
   std::vector<Colour> mcol;          // count and first of each colour (cn = {count, 1, 1})
   int *d_cmap = nullptr;             // [colour-major cell][n^3] global DoFs
+  // its inverse, for meshes that apply through local results: per DoF the positions
+  // in d_cmap that name it, ascending (so in colour order); null: coloured launches
+  int *d_touch_ptr = nullptr, *d_touch = nullptr;
   double *d_cellvert = nullptr;      // [colour-major cell][8][3] corners
   long n_cons = 0, n_masters = 0;
   long *d_cons_dof = nullptr, *d_cons_ptr = nullptr, *d_cons_mast = nullptr;  // per constraint

@@ -2157,6 +2157,12 @@ int num_sms()
 // 24 -> 24.8 / 24 -> 18.5; 25^3 Q4 (1.95M values) 46 -> 49 / 30 -> 37: hence the line.
 // The sums are the coloured apply's, bit for bit.
 constexpr long kLocalValues = 900000;  // n_cells n^3 at most
+// Mapped meshes have more and smaller colours (11 on a refined box) and gather through
+// the inverse of their map.  Applies launch by launch, constraints included, us, before
+// -> this (FP64; host-launch-bound before): Q2 26k values 42-60 -> 25-28, 286k 43 -> 26-30;
+// Q1 85k 38 -> 19-22, 968k 48 -> 36-42, 5.5M 157 -> 129-132.  At 875k values of Q2 the
+// colours' kernels alone take 41 and the two launches 46; at 3.3M 107 and 109.
+constexpr long mapped_local_values(int degree) { return degree == 1 ? 6000000 : 400000; }
 // Under a caller's capture the coloured launches stay: a graph may be replayed on any
 // stream, beside applies that use the same workspace (a solve's own capture, made with
 // fields_frozen, runs on the solve's stream).
@@ -2164,9 +2170,9 @@ template <typename Real>
 bool local_apply_ready(Op &op, const KP<Real> &k)
 {
   const Mesh &m = *op.mesh;
-  if (m.mapped || k.hsrc || k.nvec > 1 || k.zhi > k.zlo || m.NY > 65535 || m.NZ > 65535) return false;
   const long values = m.n_cells * m.n * m.n * m.n;
-  if (values > kLocalValues || op.local_slot < 0) return false;
+  if (k.hsrc || k.nvec > 1 || k.zhi > k.zlo || op.local_slot < 0) return false;
+  if (m.mapped ? !m.d_touch : values > kLocalValues || m.NY > 65535 || m.NZ > 65535) return false;
   if (!op.fields_frozen) {
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(op.stream, &st) != cudaSuccess) {
@@ -2183,7 +2189,7 @@ bool local_apply_ready(Op &op, const KP<Real> &k)
   return buf != nullptr;
 }
 
-template <int P, typename Real, int GEOM, bool NEWT = false>
+template <int P, typename Real, int GEOM, bool NEWT = false, bool MAPPED = false>
 void run_local_apply(Op &op, KP<Real> k)
 {
   Mesh &m = *op.mesh;
@@ -2192,7 +2198,7 @@ void run_local_apply(Op &op, KP<Real> k)
   const size_t smem = sizeof(Real) * warp_smem_elems<P, Real, GEOM>(NEWT ? 2 : gvel ? 1 : 0) * kWarpsPerCTA + kSmemAlign;
   if (GEOM == GEOM_GENERAL && (!k.metric || (gvel && !k.velb))) throw Error{MPDG_ERR_ARG, "coefficient stream missing"};
   k.local = static_cast<Real *>(op.d_local[op.local_slot]);
-  auto kern = warp_apply_kernel<P, Real, GEOM, false, false, false, 32, NEWT, true>;
+  auto kern = warp_apply_kernel<P, Real, GEOM, false, false, MAPPED, 32, NEWT, true>;
   static int configured_smem = -1, blocks_per_sm = 0;  // per instantiation
   if (configured_smem != (int)smem) {
     MPDG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -2201,7 +2207,14 @@ void run_local_apply(Op &op, KP<Real> k)
     configured_smem = (int)smem;
   }
   ColourRuns runs{};
-  for (int c = 0; c < 8; ++c) {
+  if constexpr (MAPPED) {
+    k.cfirst = 0;
+    runs.count[0] = (int)m.n_cells;
+    runs.m0[0] = runs.m01[0] = 1ull << 40;  // (the cell's position is not used)
+    runs.cn0[0] = runs.cn1[0] = 1;
+    for (int c = 1; c <= 8; ++c) runs.groups[c] = (int)((m.n_cells + CPW - 1) / CPW);
+  }
+  for (int c = 0; !MAPPED && c < 8; ++c) {
     const Colour &C = m.colour[c];
     colour_params(k, C);  // checks the index arithmetic
     runs.count[c] = (int)C.count;
@@ -2219,7 +2232,7 @@ void run_local_apply(Op &op, KP<Real> k)
   MPDG_LAUNCHED();
   // the gather starts as the cells' CTAs retire and waits before its first read
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)((m.NX + 127) / 128), (unsigned)m.NY, (unsigned)m.NZ);
+  cfg.gridDim = MAPPED ? dim3(grid_for(m.N, 128)) : dim3((unsigned)((m.NX + 127) / 128), (unsigned)m.NY, (unsigned)m.NZ);
   cfg.blockDim = dim3(128);
   cfg.stream = op.stream;
   cudaLaunchAttribute attr[1];
@@ -2227,7 +2240,11 @@ void run_local_apply(Op &op, KP<Real> k)
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  MPDG_CUDA(cudaLaunchKernelEx(&cfg, local_gather_kernel<P, Real>, k, runs));
+  if constexpr (MAPPED)
+    MPDG_CUDA(cudaLaunchKernelEx(&cfg, mapped_gather_kernel<Real>, k.dst, (const Real *)k.local, (const int *)m.d_touch_ptr,
+                                 (const int *)m.d_touch, k.masked_write ? k.dmask : nullptr, m.N));
+  else
+    MPDG_CUDA(cudaLaunchKernelEx(&cfg, local_gather_kernel<P, Real>, k, runs));
   MPDG_LAUNCHED();
 }
 
@@ -2542,6 +2559,16 @@ void warp_apply_degree(Op &op, const KP<Real> &k)
   const bool hang = k.hsrc != nullptr;
   if constexpr (GEOM == GEOM_GENERAL) {
     if (op.mesh->mapped) {
+      if (local_apply_ready(op, k)) {
+        switch (op.mesh->degree) {
+          case 1: run_local_apply<1, Real, GEOM, false, true>(op, k); break;
+          case 2: run_local_apply<2, Real, GEOM, false, true>(op, k); break;
+          case 3: run_local_apply<3, Real, GEOM, false, true>(op, k); break;
+          case 4: run_local_apply<4, Real, GEOM, false, true>(op, k); break;
+          default: throw Error{MPDG_ERR_UNSUPPORTED, "degree must be 1..4"};
+        }
+        return;
+      }
       switch (op.mesh->degree) {
         case 1: run_warp_apply<1, Real, GEOM, false, false, true>(op, k); break;
         case 2: run_warp_apply<2, Real, GEOM, false, false, true>(op, k); break;
