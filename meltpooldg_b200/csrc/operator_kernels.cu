@@ -2172,7 +2172,7 @@ bool local_apply_ready(Op &op, const KP<Real> &k)
   const Mesh &m = *op.mesh;
   const long values = m.n_cells * m.n * m.n * m.n;
   if (k.hsrc || k.nvec > 1 || k.zhi > k.zlo || op.local_slot < 0) return false;
-  if (m.mapped ? !m.d_touch : values > kLocalValues || m.NY > 65535 || m.NZ > 65535) return false;
+  if (m.mapped ? !m.d_touch : values > kLocalValues) return false;
   if (!op.fields_frozen) {
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(op.stream, &st) != cudaSuccess) {
@@ -2232,7 +2232,8 @@ void run_local_apply(Op &op, KP<Real> k)
   MPDG_LAUNCHED();
   // the gather starts as the cells' CTAs retire and waits before its first read
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = MAPPED ? dim3(grid_for(m.N, 128)) : dim3((unsigned)((m.NX + 127) / 128), (unsigned)m.NY, (unsigned)m.NZ);
+  const long N = MAPPED ? m.N : m.NX * m.NY * m.NZ;
+  cfg.gridDim = dim3(grid_for(N, 128));
   cfg.blockDim = dim3(128);
   cfg.stream = op.stream;
   cudaLaunchAttribute attr[1];
@@ -2242,9 +2243,9 @@ void run_local_apply(Op &op, KP<Real> k)
   cfg.numAttrs = 1;
   if constexpr (MAPPED)
     MPDG_CUDA(cudaLaunchKernelEx(&cfg, mapped_gather_kernel<Real>, k.dst, (const Real *)k.local, (const int *)m.d_touch_ptr,
-                                 (const int *)m.d_touch, k.masked_write ? k.dmask : nullptr, m.N));
+                                 (const int *)m.d_touch, k.masked_write ? k.dmask : nullptr, N));
   else
-    MPDG_CUDA(cudaLaunchKernelEx(&cfg, local_gather_kernel<P, Real>, k, runs));
+    MPDG_CUDA(cudaLaunchKernelEx(&cfg, local_gather_kernel<P, Real>, k, runs, (unsigned)N));
   MPDG_LAUNCHED();
 }
 

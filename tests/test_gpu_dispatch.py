@@ -1,0 +1,67 @@
+"""Which launches an apply takes: the forms that replace the coloured launches return
+their results, and are not slower than what they replace, on lattices that are thin
+in one or two directions.  Times are the best of several event-timed batches, with
+half as much again allowed for the machine."""
+import pytest
+
+from gpu_helpers import dev, meshes, rng
+
+pytestmark = pytest.mark.gpu
+
+SLACK = 1.5
+
+
+def best_us(f, n=20, batches=7):
+    import torch
+    f()
+    torch.cuda.synchronize()
+    e0, e1, best = torch.cuda.Event(True), torch.cuda.Event(True), float("inf")
+    for _ in range(batches):
+        e0.record()
+        for _ in range(n):
+            f()
+        e1.record()
+        torch.cuda.synchronize()
+        best = min(best, 1e3 * e0.elapsed_time(e1) / n)
+    return best
+
+
+def coloured(op, dst, src):
+    """A graph of one apply: a caller's capture keeps the coloured launches."""
+    import torch
+    g = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(g):
+        op.set_stream(torch.cuda.current_stream())
+        op.vmult(dst, src)
+    op.set_stream(None)
+    return g
+
+
+@pytest.mark.parametrize("p,nc", [(1, (1, 1, 300)), (2, (1, 70, 2)), (3, (43, 1, 1)), (4, (2, 1, 65)), (2, (3, 33, 7))])
+def test_thin_lattices_in_two_launches_equal_the_colours(cuda, p, nc):
+    """Rows that do not fill a block of the gather, blocks that end inside a row."""
+    import torch
+    import meltpooldg_b200 as M
+    gm, _ = meshes(nc, p, 0.1, seed=3, mask=M.boundary_mask(nc, p, faces=[(0, 0), (2, 1)]))
+    op = M.HeatDiffuseOperator(gm, 1e-3, precisions=("fp64", "fp32"))
+    for dtype in (torch.float64, torch.float32):
+        s = dev(rng(4).uniform(-1, 1, gm.n_dofs), dtype)
+        two, eight = torch.full_like(s, float("nan")), torch.full_like(s, float("nan"))
+        op.vmult(two, s)
+        coloured(op, eight, s).replay()
+        torch.cuda.synchronize()
+        assert torch.equal(two, eight)
+
+
+@pytest.mark.parametrize("p,nc", [(1, (2, 170, 180)), (2, (2, 90, 100))])
+def test_two_launches_on_thin_lattices_are_not_slower_than_the_colours(cuda, p, nc):
+    import torch
+    import meltpooldg_b200 as M
+    gm, _ = meshes(nc, p, 0.1, seed=3)
+    op = M.HeatDiffuseOperator(gm, 1e-3)
+    s = dev(rng(4).uniform(-1, 1, gm.n_dofs))
+    d = torch.empty_like(s)
+    two = best_us(lambda: op.vmult(d, s))
+    eight = best_us(coloured(op, d, s).replay)
+    assert two < SLACK * eight, (two, eight)
