@@ -65,3 +65,17 @@ def test_two_launches_on_thin_lattices_are_not_slower_than_the_colours(cuda, p, 
     two = best_us(lambda: op.vmult(d, s))
     eight = best_us(coloured(op, d, s).replay)
     assert two < SLACK * eight, (two, eight)
+
+
+def test_long_lattices_are_not_slower_than_the_colours(cuda):
+    """4,000 cell layers: what the host does for one launch does not grow with them."""
+    import torch
+    import meltpooldg_b200 as M
+    gm, _ = meshes((2, 2, 4000), 1, 0.0)
+    op = M.HeatDiffuseOperator(gm, 1e-3)
+    s = dev(rng(4).uniform(-1, 1, gm.n_dofs))
+    d = torch.empty_like(s)
+    default = best_us(lambda: op.vmult(d, s))
+    op.set_schedule(1, False, "fp64", overlap_colours=True, lane_cells=0)
+    eight = best_us(coloured(op, d, s).replay)
+    assert default < SLACK * eight, (default, eight)
