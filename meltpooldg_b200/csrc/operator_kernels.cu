@@ -2172,6 +2172,7 @@ bool local_apply_ready(Op &op, const KP<Real> &k)
   const Mesh &m = *op.mesh;
   const long values = m.n_cells * m.n * m.n * m.n;
   if (k.hsrc || k.nvec > 1 || k.zhi > k.zlo || op.local_slot < 0) return false;
+  if (!m.mapped && (m.nc[0] > 1) + (m.nc[1] > 1) + (m.nc[2] > 1) < 2) return false;  // two colours at most
   if (m.mapped ? !m.d_touch : values > kLocalValues) return false;
   if (!op.fields_frozen) {
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
@@ -2339,11 +2340,11 @@ void run_warp_apply(Op &op, KP<Real> k)
   }
 }
 
-// the band apply serves uniform lattices with constant coefficients, no
-// hanging DoFs and a velocity that is a product along the axes.  The vortex
-// has (P+1)^2 coefficients of its own per x-unit; they are built for degrees 1
-// and 2.
-bool band_eligible(const Op &op)
+// operators that are sums of line products: uniform lattices with constant
+// coefficients, no hanging DoFs and a velocity that is a product along the axes.
+// The vortex has (P+1)^2 coefficients of its own per x-unit; they are built for
+// degrees 1 and 2.
+bool band_form(const Op &op)
 {
   const Mesh &m = *op.mesh;
   if (!m.uniform || m.mapped || op.hang_src || supg(op) || uses_kT(op)) return false;
@@ -2352,12 +2353,47 @@ bool band_eligible(const Op &op)
          (op.d.vel_kind == MPDG_VEL_VORTEX && m.degree <= 2);
 }
 
-// whether the schedule of one precision runs it: by default, and for degrees
-// 1 and 2 where lane_cells asks for it
+// whether the band apply is built for it.  The rotation's second pair of products
+// spills at degree 4 (FP64 2.1 KB a lane: 64^3 546 us, warp apply 428; 24^3 70, 34;
+// FP32 28^3 39, 32): the warp apply keeps it.
+bool band_serves(const Op &op)
+{
+  return band_form(op) && !(op.d.vel_kind == MPDG_VEL_ROTATION && op.mesh->degree >= 4);
+}
+
+// whether it is the faster apply.  A strip costs the same however few of its x-units
+// and rows hold cells, so the line is the share that do; where the warp apply costs a
+// cell less (low degrees) a smaller share is enough.  FP64 without a velocity, us, band
+// and the other launches, below and above the line:
+//   Q1 0.08  4x16x4000 (0.06) 36, 27       10x10x60 (0.15) 5.1, 7.7   256^3 113, 1240
+//   Q2 0.20  4x16x4000 (0.13) 101, 81      16x4x1000 (0.43) 20, 28    128^3 105, 619
+//   Q3 0.43  4x16x1000 (0.19) 81, 46       9x28x49 (0.43) 16, 25      64^3 82, 179
+//   Q4 0.65  9x28x49 (0.62) 31, 28         19x34x50 (0.66) 51, 56     64^3 235, 397
+// Small lattices are latency: at degrees 1 and 2 one launch is sooner than two down to a
+// share of 0.03 (Q1 4x100x4 4.9, 8.2, Q2 6x45x11 6.2, 8.2; single cells in x and y, Q2
+// 1x1x1000 vortex 14, 7); at degrees 3 and 4 a plane of a strip takes 2 us (Q3 16^3 12.3,
+// 10.3, 20^3 12.3, 15.1; Q4 16^3 20.5, 17.2, 10x10x60 21.3, 24.6).  The rotation at
+// degree 3 (576 bytes of spills): 40^3 (0.65) 53, 52, 1000x4x4 26, 23, 45x39x52 (0.73)
+// 59, 71, 64^3 146, 189.
+bool band_pays(const Op &op)
+{
+  const Mesh &m = *op.mesh;
+  const int P = m.degree, nxu = 63 / P - 1;  // (BandShape::nxu)
+  const long values = m.n_cells * m.n * m.n * m.n;
+  const double strips = (m.nc[0] + nxu) / nxu;
+  const double fill = m.nc[0] / (strips * nxu) * m.nc[1] / (m.nc[1] + 1.0);
+  if (P == 3 && op.d.vel_kind == MPDG_VEL_ROTATION) return fill >= 0.70 && m.nc[1] >= 16 && values > 1500000;
+  if (P == 1) return fill >= (values <= 100000 ? 0.03 : 0.08);
+  if (P == 2) return fill >= (values <= 100000 ? 0.03 : 0.20);
+  return P == 3 ? fill >= 0.43 && values > 250000 : fill >= 0.65 && values > 500000;
+}
+
+// whether the schedule of one precision runs it: by default where it is faster, and
+// for degrees 1 and 2 where lane_cells asks for it
 bool band_scheduled(const Op &op, int precision)
 {
   const ApplySchedule &s = op.sched[precision];
-  return band_eligible(op) && (s.band || (s.lane && op.mesh->degree <= 2));
+  return band_serves(op) && (s.band ? band_pays(op) : (s.lane && op.mesh->degree <= 2));
 }
 
 // element matrices of degree p on [0,1]: mass, stiffness, advection
@@ -2462,6 +2498,10 @@ void run_band(Op &op, const KP<Real> &k, bool add)
   b.nxu = (ux + b.ntx - 1) / b.ntx;
   // fewer warps per CTA while the chip has CTAs to spare
   b.warps = BS::warps;
+  // FP64 Q2: three warps where a fourth would stand idle in a sixth of the CTA's rows
+  // (16x4x4000, five y-units: 51 -> 41 us, vortex 75 -> 58; FP32 31 -> 40 with five of
+  // eight, Q3 42 -> 52: not there)
+  if (P == 2 && BS::f64 && 6 * ((uy + 2) / 3 * 3) <= 5 * ((uy + 3) / 4 * 4)) b.warps = 3;
   while (b.warps > 1 && (long)b.ntx * ((uy + b.warps - 1) / b.warps) * m.nc[2] < num_sms()) b.warps /= 2;
   b.nty = (uy + b.warps - 1) / b.warps;
   constexpr size_t warp_smem = sizeof(Real2) * BS::warp_pairs(VK == BAND_VORTEX);
@@ -2506,7 +2546,7 @@ template <int P, typename Real>
 void band_apply_velocity(Op &op, const KP<Real> &k, bool add)
 {
   if (k.vel_kind == MPDG_VEL_ROTATION) {
-    run_band<P, Real, BAND_ROTATION>(op, k, add);
+    if constexpr (P <= 3) run_band<P, Real, BAND_ROTATION>(op, k, add);
   } else if (k.vel_kind == MPDG_VEL_VORTEX) {
     if constexpr (P <= 2) run_band<P, Real, BAND_VORTEX>(op, k, add);
   } else {
@@ -3286,7 +3326,7 @@ void autotune_apply(Op &op, int precision, int reps, ApplySchedule &best, double
   // constant-coefficient path with an in-kernel velocity
   const bool lane_ok = m.uniform && !m.mapped && !op.fine && (m.degree == 1 || m.degree == 2) &&
                        plain_warp_apply(op) && !uses_kT(op) && op.d.vel_kind != MPDG_VEL_NODAL;
-  const int lane_max = lane_ok && band_eligible(op) ? 1 : 0;
+  const int lane_max = lane_ok && band_serves(op) ? 1 : 0;
   for (int S : {1, 2}) {
     if (S > 1 && (S > m.nc[2] / 2 || m.mapped || op.fine)) continue;
     for (int h = 0; h <= (stream ? 1 : 0); ++h)
@@ -3449,7 +3489,7 @@ void launch_rhs(Op &op, double *dst, const double *src, const double *heat_sourc
     // tested with grad N (advection_diffusion_operator.cpp:336-346)
     // 128^3 Q2 vortex: 1,600 us by the block kernel in eight colours
     if (supg(op)) dispatch_degree<double, MODE_SUPG, false>(op, k);
-    else if (band_eligible(op)) band_apply<double>(op, k, true);
+    else if (band_serves(op)) band_apply<double>(op, k, true);
     else dispatch_degree<double, MODE_LINEAR, false>(op, k);
   }
   // integrate_scatter through the constraints: the constrained rows go to their masters
@@ -3593,7 +3633,7 @@ void launch_block_diagonal(Op &op, double *diag)
   check_law_fields(op, k);
   // 128^3 Q2 vortex: 1,470 us by the cells' element diagonals in eight colours; a
   // DoF's diagonal is a handful of products on such a lattice
-  const bool band = band_eligible(op) && m.NY <= 65535;
+  const bool band = band_form(op) && m.NY <= 65535;
   if (!band) MPDG_CUDA(cudaMemsetAsync(diag, 0, sizeof(double) * m.N_own, op.stream));
 
   switch (band ? -m.degree : m.degree) {

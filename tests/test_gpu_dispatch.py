@@ -2,9 +2,11 @@
 their results, and are not slower than what they replace, on lattices that are thin
 in one or two directions.  Times are the best of several event-timed batches, with
 half as much again allowed for the machine."""
+import numpy as np
 import pytest
 
-from gpu_helpers import dev, meshes, rng
+from gpu_helpers import dev, meshes, relerr, rng
+from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
 
@@ -79,3 +81,45 @@ def test_long_lattices_are_not_slower_than_the_colours(cuda):
     op.set_schedule(1, False, "fp64", overlap_colours=True, lane_cells=0)
     eight = best_us(coloured(op, d, s).replay)
     assert default < SLACK * eight, (default, eight)
+
+
+@pytest.mark.parametrize("p,nc,vel", [(4, (8, 60, 40), ("rotation", 0.8)), (4, (24, 24, 24), ("rotation", 0.8)),
+                                      (3, (2, 100, 100), None), (4, (2, 100, 100), None), (3, (4, 16, 500), None),
+                                      (2, (4, 4, 4000), ("rotation", 0.8)), (1, (4, 16, 4000), "vortex"),
+                                      (4, (1, 1, 100), None), (3, (30, 1, 1), ("rotation", 0.8))])
+def test_the_default_apply_is_not_slower_than_the_colours(cuda, p, nc, vel):
+    """Uniform lattices whose strips of the band apply would stay nearly empty, or whose
+    products spill: the default takes the launches that are faster there."""
+    import torch
+    import meltpooldg_b200 as M
+    gm, _ = meshes(nc, p, 0.0)
+    op = M.AdvectionDiffusionOperator(gm, 1e-3, theta=0.5, diffusivity=1e-2, velocity=vel)
+    s = dev(rng(4).uniform(-1, 1, gm.n_dofs))
+    d, e = torch.empty_like(s), torch.empty_like(s)
+    default = best_us(lambda: op.vmult(d, s))
+    op.set_schedule(1, False, "fp64", overlap_colours=True, cta_cell_groups=p in (2, 4), lane_cells=0)
+    eight = best_us(coloured(op, e, s).replay)
+    assert (d - e).abs().max() <= 1e-13 * e.abs().max()
+    assert default < SLACK * eight, (default, eight)
+
+
+@pytest.mark.parametrize("p,nc", [(3, (20, 20, 10)), (3, (19, 3, 70)), (4, (13, 20, 16)), (4, (27, 10, 16))])
+@pytest.mark.parametrize("mask", ["none", "some_faces", "scattered"])
+def test_band_apply_of_degrees_3_and_4_at_its_smallest_sizes(cuda, p, nc, mask):
+    import torch
+    import meltpooldg_b200 as M
+    m = {"none": lambda: None, "some_faces": lambda: M.boundary_mask(nc, p, faces=[(0, 1), (2, 0)]),
+         "scattered": lambda: (rng(5).uniform(size=int(np.prod([n * p + 1 for n in nc]))) < 0.1).astype(np.uint8)}[mask]()
+    gm, om = meshes(nc, p, 0.0, mask=m, hi=(1.0, 0.8, 1.3))
+    op = M.AdvectionDiffusionOperator(gm, 1e-3, theta=0.5, diffusivity=1e-2, velocity=(0.7, -0.4, 0.25),
+                                      precisions=("fp64", "fp32"))
+    oop = O.Operator(O.ADVDIFF, 1e-3, theta=0.5, diffusivity=1e-2, dirichlet=m, vel_kind=O.VEL_CONST,
+                     vel_param=(0.7, -0.4, 0.25))
+    src = rng(70 + p).uniform(-1, 1, gm.n_dofs)
+    ref = O.vmult(om, oop, src)
+    for dtype, tol in ((torch.float64, 1e-12), (torch.float32, 2e-5)):
+        out = torch.full((gm.n_dofs,), float("nan"), dtype=dtype, device="cuda")
+        before = M.kernel_launches()
+        op.vmult(out, dev(src, dtype))
+        assert M.kernel_launches() - before == 1
+        assert relerr(out.cpu().numpy().astype(np.float64), ref) < tol
