@@ -2573,19 +2573,23 @@ void band_apply(Op &op, const KP<Real> &k, bool add = false)
   }
 }
 
-// the diagonal of an operator the band apply serves (every DoF; constrained ones too)
+// the diagonal of an operator of line products (every DoF; constrained ones too)
 template <int P>
 void run_band_diag(Op &op, const KP<double> &k)
 {
   const Mesh &m = *op.mesh;
-  const dim3 grid((unsigned)((m.NX + 127) / 128), (unsigned)m.NY, (unsigned)std::min(m.NZ, 16L));
+  const unsigned blocks = grid_for(m.NX * m.NY, 128);
+  // 16 blocks per SM, at least four planes to a column's factors
+  const long chunks = std::max(1L, std::min((m.NZ + 3) / 4, 16L * num_sms() / blocks));
+  const int zlen = (int)((m.NZ + chunks - 1) / chunks);
+  const dim3 grid(blocks, (unsigned)((m.NZ + zlen - 1) / zlen));
   if (k.vel_kind == MPDG_VEL_ROTATION) {
-    band_diag_kernel<P, double, BAND_ROTATION><<<grid, 128, 0, op.stream>>>(band_params<P, double, BAND_ROTATION>(op, k));
+    band_diag_kernel<P, double, BAND_ROTATION><<<grid, 128, 0, op.stream>>>(band_params<P, double, BAND_ROTATION>(op, k), zlen);
   } else if (k.vel_kind == MPDG_VEL_VORTEX) {
     if constexpr (P <= 2)
-      band_diag_kernel<P, double, BAND_VORTEX><<<grid, 128, 0, op.stream>>>(band_params<P, double, BAND_VORTEX>(op, k));
+      band_diag_kernel<P, double, BAND_VORTEX><<<grid, 128, 0, op.stream>>>(band_params<P, double, BAND_VORTEX>(op, k), zlen);
   } else {
-    band_diag_kernel<P, double, BAND_PLAIN><<<grid, 128, 0, op.stream>>>(band_params<P, double, BAND_PLAIN>(op, k));
+    band_diag_kernel<P, double, BAND_PLAIN><<<grid, 128, 0, op.stream>>>(band_params<P, double, BAND_PLAIN>(op, k), zlen);
   }
   MPDG_LAUNCHED();
 }
@@ -3633,7 +3637,7 @@ void launch_block_diagonal(Op &op, double *diag)
   check_law_fields(op, k);
   // 128^3 Q2 vortex: 1,470 us by the cells' element diagonals in eight colours; a
   // DoF's diagonal is a handful of products on such a lattice
-  const bool band = band_form(op) && m.NY <= 65535;
+  const bool band = band_form(op);
   if (!band) MPDG_CUDA(cudaMemsetAsync(diag, 0, sizeof(double) * m.N_own, op.stream));
 
   switch (band ? -m.degree : m.degree) {

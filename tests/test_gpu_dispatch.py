@@ -123,3 +123,20 @@ def test_band_apply_of_degrees_3_and_4_at_its_smallest_sizes(cuda, p, nc, mask):
         op.vmult(out, dev(src, dtype))
         assert M.kernel_launches() - before == 1
         assert relerr(out.cpu().numpy().astype(np.float64), ref) < tol
+
+
+@pytest.mark.parametrize("p,nc,vel", [(2, (4, 2000, 4), "vortex"), (2, (64, 64, 64), "vortex"), (2, (100, 100, 2), "vortex"),
+                                      (4, (32, 32, 32), ("rotation", 0.8)), (3, (1, 1, 1000), None),
+                                      (4, (4, 1000, 4), ("rotation", 0.8))])
+def test_diagonal_from_line_factors_is_not_slower_than_from_the_cells(cuda, p, nc, vel):
+    """The same lattice as general cells takes the cells' element diagonals."""
+    import torch
+    import meltpooldg_b200 as M
+    d, us = [], []
+    for geometry in ("auto", "general"):
+        gm, _ = meshes(nc, p, 0.0, geometry=geometry)
+        op = M.AdvectionDiffusionOperator(gm, 1e-3, theta=0.5, diffusivity=1e-2, velocity=vel)
+        d.append(torch.empty(gm.n_dofs, dtype=torch.float64, device="cuda"))
+        us.append(best_us(lambda: op.compute_diagonal(d[-1])))
+    assert (d[0] - d[1]).abs().max() <= 1e-12 * d[1].abs().max()
+    assert us[0] < SLACK * us[1], us
