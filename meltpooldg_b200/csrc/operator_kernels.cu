@@ -2361,6 +2361,14 @@ bool band_serves(const Op &op)
   return band_form(op) && !(op.d.vel_kind == MPDG_VEL_ROTATION && op.mesh->degree >= 4);
 }
 
+// the share of the band apply's strips (x-units and rows) that holds cells
+double strip_fill(const Mesh &m)
+{
+  const int nxu = 63 / m.degree - 1;  // (BandShape::nxu)
+  const double strips = (m.nc[0] + nxu) / nxu;
+  return m.nc[0] / (strips * nxu) * m.nc[1] / (m.nc[1] + 1.0);
+}
+
 // whether it is the faster apply.  A strip costs the same however few of its x-units
 // and rows hold cells, so the line is the share that do; where the warp apply costs a
 // cell less (low degrees) a smaller share is enough.  FP64 without a velocity, us, band
@@ -2378,10 +2386,9 @@ bool band_serves(const Op &op)
 bool band_pays(const Op &op)
 {
   const Mesh &m = *op.mesh;
-  const int P = m.degree, nxu = 63 / P - 1;  // (BandShape::nxu)
+  const int P = m.degree;
   const long values = m.n_cells * m.n * m.n * m.n;
-  const double strips = (m.nc[0] + nxu) / nxu;
-  const double fill = m.nc[0] / (strips * nxu) * m.nc[1] / (m.nc[1] + 1.0);
+  const double fill = strip_fill(m);
   if (P == 3 && op.d.vel_kind == MPDG_VEL_ROTATION) return fill >= 0.70 && m.nc[1] >= 16 && values > 1500000;
   if (P == 1) return fill >= (values <= 100000 ? 0.03 : 0.08);
   if (P == 2) return fill >= (values <= 100000 ? 0.03 : 0.20);
@@ -3491,9 +3498,13 @@ void launch_rhs(Op &op, double *dst, const double *src, const double *heat_sourc
     k.full_tangent = 0;
     // SUPG: + tau_K u (phi_old/dt - (1-theta) u.grad phi_old + (1-theta) D lap phi_old)
     // tested with grad N (advection_diffusion_operator.cpp:336-346)
-    // 128^3 Q2 vortex: 1,600 us by the block kernel in eight colours
+    // 128^3 Q2 vortex: 1,600 us by the block kernel in eight colours, 200 as line products;
+    // not on strips that are nearly empty, us, line products and cells: Q2 1x1x4000
+    // (share 0.02) 24, 15, 4x4x4000 (0.11) 46, 80; Q3 4x4x4000 (0.16) 186, 131, 4x4000x4
+    // (0.20) 96, 131; Q4 4x4x4000 (0.23) 425, 249, 4x4000x4 (0.29) 204, 247
+    static constexpr double least[kMaxDegree + 1] = {0, 0.03, 0.03, 0.18, 0.28};
     if (supg(op)) dispatch_degree<double, MODE_SUPG, false>(op, k);
-    else if (band_serves(op)) band_apply<double>(op, k, true);
+    else if (band_serves(op) && strip_fill(*op.mesh) >= least[op.mesh->degree]) band_apply<double>(op, k, true);
     else dispatch_degree<double, MODE_LINEAR, false>(op, k);
   }
   // integrate_scatter through the constraints: the constrained rows go to their masters

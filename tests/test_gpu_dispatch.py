@@ -140,3 +140,21 @@ def test_diagonal_from_line_factors_is_not_slower_than_from_the_cells(cuda, p, n
         us.append(best_us(lambda: op.compute_diagonal(d[-1])))
     assert (d[0] - d[1]).abs().max() <= 1e-12 * d[1].abs().max()
     assert us[0] < SLACK * us[1], us
+
+
+@pytest.mark.parametrize("p,nc", [(2, (1, 1, 2000)), (3, (1, 1, 1000)), (4, (1, 1, 1000)), (4, (4, 4, 2000)), (3, (20, 9, 4)), (4, (13, 6, 5))])
+def test_rhs_as_line_products_is_not_slower_than_from_the_cells(cuda, p, nc):
+    """The same lattice as general cells takes the cells' block kernel."""
+    import torch
+    import meltpooldg_b200 as M
+    d, us = [], []
+    for geometry in ("auto", "general"):
+        gm, _ = meshes(nc, p, 0.0, geometry=geometry, mask=M.boundary_mask(nc, p, faces=[(0, 0)]))
+        op = M.AdvectionDiffusionOperator(gm, 1e-3, theta=0.5, diffusivity=1e-2, velocity=(0.3, 0.1, -0.2))
+        phi = dev(rng(8).uniform(-1, 1, gm.n_dofs))
+        d.append(torch.zeros(gm.n_dofs, dtype=torch.float64, device="cuda"))
+        op.create_rhs(d[-1], phi)
+        spare = torch.zeros_like(phi)
+        us.append(best_us(lambda: op.create_rhs(spare, phi)))
+    assert (d[0] - d[1]).abs().max() <= 1e-12 * d[1].abs().max()
+    assert us[0] < SLACK * us[1], us
