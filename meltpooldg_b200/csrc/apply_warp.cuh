@@ -441,6 +441,11 @@ __global__ void __launch_bounds__(128) mapped_gather_kernel(Real *dst, const Rea
   dst[g] = masked ? Real(0) : s;
 }
 
+// (the other applies carry no runs: 264 bytes of parameters less per launch, 1 us of the
+// 23 that the host takes for an apply's eight)
+struct NoRuns {
+};
+
 template <int P, typename Real>
 struct WOcc {
   static constexpr int min_blocks = (sizeof(Real) == 8) ? (P == 4 ? 3 : P == 3 ? 4 : P == 2 ? 5 : 6)
@@ -465,7 +470,7 @@ struct WOcc {
 template <int P, typename Real, int GEOM, bool HANG = false, bool MULTI = false, bool MAPPED = false,
           int GROUP = 32, bool NEWT = false, bool LOCAL = false>
 __global__ void __launch_bounds__(kWarpsPerCTA * 32, WOcc<P, Real>::min_blocks)
-    warp_apply_kernel(const KP<Real> p, int *err, const ColourRuns runs)
+    warp_apply_kernel(const KP<Real> p, int *err, const std::conditional_t<LOCAL, ColourRuns, NoRuns> runs)
 {
   static_assert(!(HANG && MULTI), "the multi-vector apply has no hanging-node path");
   static_assert(!(MAPPED && (HANG || MULTI || GEOM != GEOM_GENERAL)), "mapped meshes: general geometry, one vector");
@@ -512,7 +517,8 @@ __global__ void __launch_bounds__(kWarpsPerCTA * 32, WOcc<P, Real>::min_blocks)
   Real *t1 = tiles + L::t0_elems + s_sub * L::sc1;
   // DoF offsets are 32-bit: the launcher checks that the lattice has < 2^32 DoFs
   const unsigned NXu = (unsigned)p.NX, NYu = (unsigned)p.NY, zs = NXu * NYu;
-  const int count = LOCAL ? runs.groups[8] * CPW : (int)p.ccount;  // LOCAL: groups of all colours
+  int count = (int)p.ccount;
+  if constexpr (LOCAL) count = runs.groups[8] * CPW;  // groups of all colours
   const int gstride = gridDim.x * GPC;
   unsigned phase = 0;
 

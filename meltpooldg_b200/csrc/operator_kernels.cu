@@ -2317,7 +2317,7 @@ void run_warp_apply(Op &op, KP<Real> k)
       attr[0].val.programmaticStreamSerializationAllowed = 1;
       cfg.attrs = attr;
       cfg.numAttrs = pdl ? 1 : 0;
-      MPDG_CUDA(cudaLaunchKernelEx(&cfg, kern, k, op.d_err, ColourRuns{}));
+      MPDG_CUDA(cudaLaunchKernelEx(&cfg, kern, k, op.d_err, NoRuns{}));
       MPDG_LAUNCHED();
       ++launched;
     }
