@@ -559,7 +559,7 @@ void build_mapped_mesh(Mesh &m, const mpdg_mapped_mesh_desc &d)
   size_t &B = m.device_bytes;
   m.d_cmap = upload(cmap, B);
   m.d_cell_first = upload(cfirst, B);
-  if (n_col > 2 && (long)cmap.size() <= mapped_local_values(p)) {
+  if (n_col > 2 && (long)cmap.size() <= mapped_local_values(p, n_col)) {
     std::vector<int> ptr((size_t)N + 1, 0), touch(cmap.size());
     for (const int g : cmap) ++ptr[g + 1];
     for (long g = 0; g < N; ++g) ptr[g + 1] += ptr[g];

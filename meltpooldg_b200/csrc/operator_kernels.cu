@@ -2150,19 +2150,33 @@ int num_sms()
 }
 
 // Small lattices apply in two launches -- all cells into local results, then a
-// gather per DoF -- instead of eight colours, whose launches take 23 us whatever the
-// size; the extra pass over n^3 values per cell stays in the L2.  Measured (general
-// cells, FP64 / FP32, us, coloured -> this): 8^3 Q2 24 -> 8.3 / 23 -> 7.8, 20^3 Q3
-// 26 -> 16.5 / 27 -> 14.4, 16^3 Q4 24 -> 19.8 / 23 -> 15.3, 40x32x24 Q2 (829k values)
-// 24 -> 24.8 / 24 -> 18.5; 25^3 Q4 (1.95M values) 46 -> 49 / 30 -> 37: hence the line.
-// The sums are the coloured apply's, bit for bit.
-constexpr long kLocalValues = 900000;  // n_cells n^3 at most
-// Mapped meshes have more and smaller colours (11 on a refined box) and gather through
-// the inverse of their map.  Applies launch by launch, constraints included, us, before
-// -> this (FP64; host-launch-bound before): Q2 26k values 42-60 -> 25-28, 286k 43 -> 26-30;
-// Q1 85k 38 -> 19-22, 968k 48 -> 36-42, 5.5M 157 -> 129-132.  At 875k values of Q2 the
-// colours' kernels alone take 41 and the two launches 46; at 3.3M 107 and 109.
-constexpr long mapped_local_values(int degree) { return degree == 1 ? 6000000 : 400000; }
+// gather per DoF -- instead of eight colours, whose launches take 19-23 us whatever the
+// size; the extra pass over n^3 values per cell stays in the L2.  The sums are the
+// coloured apply's, bit for bit.  Measured, us, this and coloured (general cells unless
+// said otherwise), below and above the lines:
+//   FP64        Q1 40^3 (512k values) 15, 23   Q4 4x4x300 (600k) 20.5, 20-22  Q2 30^3 (729k) 22.6, 19.6
+//   FP64 uniform, velocity vector              Q4 4x4x300 18.6, 22.5          Q2 2x128x128 (885k) 22.6, 22.6
+//   FP32        Q4 4x16x100 (800k) 18.6, 22.1  Q2 2x128x128 20.4, 22.2        Q4 25^3 (1.95M) 37, 30
+// Within a solve an apply follows another kernel of 3-8 us, and a round trip in GMRES, so
+// two launches pay for longer: Newton step of Q2 gas/liquid/solid heat at 829k values
+// 3.94 ms, 4.08; CG Q2 829k 6.11, 6.12, Q3 682k 6.6, 7.2; but Q4 512k 7.1, 7.4, 729k 8.8, 8.5.
+template <typename Real>
+long local_values(const Op &op)
+{
+  const Mesh &m = *op.mesh;
+  if (sizeof(Real) == 4 || m.uniform) return 900000;
+  return !op.fields_frozen ? 550000 : m.degree == 4 ? 600000 : 900000;
+}
+// Mapped meshes gather through the inverse of their map; most have more and smaller
+// colours (11 on a refined box, 17-20 where the cells come in no order).  Us, this and
+// coloured, FP64: Q2 26k values 25-28, 42-60, 286k 26-30, 43 (11 colours), at 875k the
+// kernels alone 46, 41; Q3, Q4 343-373k 13-14, 20 (8 colours).  Q1, 11 colours, 968k
+// 36-42, 48, 5.5M 129-132, 157; 8 colours 885k 21.6, 21.4, and from there on more: 3M
+// FP32 38.8, 33.8, 5.8M FP64 102.5, 99.0.
+constexpr long mapped_local_values(int degree, int colours)
+{
+  return degree > 1 ? 400000 : colours > 8 ? 6000000 : 900000;
+}
 // Under a caller's capture the coloured launches stay: a graph may be replayed on any
 // stream, beside applies that use the same workspace (a solve's own capture, made with
 // fields_frozen, runs on the solve's stream).
@@ -2173,7 +2187,7 @@ bool local_apply_ready(Op &op, const KP<Real> &k)
   const long values = m.n_cells * m.n * m.n * m.n;
   if (k.hsrc || k.nvec > 1 || k.zhi > k.zlo || op.local_slot < 0) return false;
   if (!m.mapped && (m.nc[0] > 1) + (m.nc[1] > 1) + (m.nc[2] > 1) < 2) return false;  // two colours at most
-  if (m.mapped ? !m.d_touch : values > kLocalValues) return false;
+  if (m.mapped ? !m.d_touch : values > local_values<Real>(op)) return false;
   if (!op.fields_frozen) {
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(op.stream, &st) != cudaSuccess) {

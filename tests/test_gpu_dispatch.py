@@ -158,3 +158,43 @@ def test_rhs_as_line_products_is_not_slower_than_from_the_cells(cuda, p, nc):
         us.append(best_us(lambda: op.create_rhs(spare, phi)))
     assert (d[0] - d[1]).abs().max() <= 1e-12 * d[1].abs().max()
     assert us[0] < SLACK * us[1], us
+
+
+def launches(f):
+    import meltpooldg_b200 as M
+    f()
+    before = M.kernel_launches()
+    f()
+    return M.kernel_launches() - before
+
+
+def test_two_launches_up_to_the_measured_sizes(cuda):
+    """General cells: FP64 up to 550,000 local values outside a solve, FP32 up to 900,000."""
+    import torch
+    import meltpooldg_b200 as M
+    for nc, fp64 in (((28, 28, 24), 2), ((32, 32, 24), 8)):
+        gm, _ = meshes(nc, 2, 0.1, seed=3)
+        op = M.HeatDiffuseOperator(gm, 1e-3, precisions=("fp64", "fp32"))
+        for dtype, n in ((torch.float64, fp64), (torch.float32, 2)):
+            s = dev(rng(4).uniform(-1, 1, gm.n_dofs), dtype)
+            d = torch.empty_like(s)
+            assert launches(lambda: op.vmult(d, s)) == n
+
+
+@pytest.mark.parametrize("n,order,count", [(40, "lexicographic", 2), (50, "lexicographic", 8), (50, "shuffled", 2)])
+def test_mapped_q1_in_two_launches_where_its_colours_are_many(cuda, n, order, count):
+    import torch
+    import meltpooldg_b200 as M
+    i, j, k = (a.reshape(-1) for a in np.meshgrid(*[np.arange(n)] * 3, indexing="ij"))
+    cell = np.stack([k, j, i], 1)
+    corner = np.stack([(np.arange(8) >> d) & 1 for d in range(3)], 1)
+    at = cell[:, None] + corner[None]
+    dofs = at @ np.array([1, n + 1, (n + 1) ** 2])
+    if order == "shuffled":
+        p = rng(2).permutation(len(cell))
+        at, dofs = at[p], dofs[p]
+    gm = M.MappedMesh(at / n, dofs, (n + 1) ** 3, 1)
+    op = M.HeatDiffuseOperator(gm, 1e-3)
+    s = dev(rng(4).uniform(-1, 1, gm.n_dofs))
+    d = torch.empty_like(s)
+    assert launches(lambda: op.vmult(d, s)) == count
