@@ -290,14 +290,16 @@ mpdg_status mpdg_vmult_multi(mpdg_op *op, int n_vectors, double *const *dst, con
  * dst wait for it; cta_cell_groups lets the four warps of a CTA share their
  * cells (5 Q4 cells or 14 Q2 cells per 128 threads instead of 4 or 12, so
  * fewer lanes idle; the tile exchanges become CTA barriers), for degrees 2
- * and 4 on lattice meshes.  lane_cells (uniform lattices of degree 1 or 2,
- * constant coefficients, velocities other than MPDG_VEL_NODAL) selects the band
- * apply, which applies the operator as sums of products of line matrices; it is
- * the default there, and on uniform lattices of degree 3 and 4 until a schedule is
- * set.  Results are identical for every schedule without lane_cells, and agree
- * with them to rounding with it; lattices of at most 900,000 local values (cells
- * times (degree + 1)^3) run in two launches whatever the schedule says, with the
- * same bits.  No reference
+ * and 4 on lattice meshes.  lane_cells chooses the form of the apply: 0 the
+ * coloured launches that the other fields describe; 1, the default, the band
+ * apply (one launch, sums of products of line matrices) on uniform lattices with
+ * constant coefficients and two launches (all cells into local results, one
+ * gather per DoF) on small lattices and mapped meshes, each where it is the
+ * faster, else the coloured launches; 2 the band apply wherever it is built (no,
+ * a constant or a rotating velocity, the vortex at degrees 1 and 2, the rotation
+ * up to degree 3).  Captures by the caller keep the coloured launches of small
+ * meshes.  Results are identical for every schedule that does not take the band
+ * apply, and agree with them to rounding where it does.  No reference
  * counterpart: the schedule of deal.II's MatrixFree::cell_loop
  * (heat_diffuse_operator.cpp:183) is internal to it. */
 typedef struct {
@@ -305,7 +307,7 @@ typedef struct {
   int l2_evict_first;   /* 0 or 1 */
   int overlap_colours;  /* 0 or 1 */
   int cta_cell_groups;  /* 0 or 1 */
-  int lane_cells;       /* 0: warp apply; 1, 2: band apply */
+  int lane_cells;       /* 0, 1 or 2, see above */
 } mpdg_schedule;
 mpdg_status mpdg_op_set_schedule(mpdg_op *op, int precision, const mpdg_schedule *schedule);
 mpdg_status mpdg_op_get_schedule(mpdg_op *op, int precision, mpdg_schedule *schedule);

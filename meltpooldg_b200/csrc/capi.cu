@@ -257,11 +257,6 @@ mpdg_status mpdg_op_create(mpdg_mesh *mesh, const mpdg_op_desc *desc, mpdg_op **
     // 64^3 Q4 FP64 0.490 -> 0.485 ms; Q4 FP32 0.294 -> 0.299 ms, kept on warps)
     o.sched[MPDG_FP64].cta = (mm.degree == 2 || mm.degree == 4) ? 1 : 0;
     o.sched[MPDG_FP32].cta = mm.degree == 2 ? 1 : 0;
-    // the band apply serves uniform lattices of degree 1 and 2 by default; the
-    // schedule reports it as lane_cells (degrees 3 and 4: not a schedule option)
-    const int lane_default = mm.degree <= 2 ? 1 : 0;
-    o.sched[MPDG_FP64].lane = lane_default;
-    o.sched[MPDG_FP32].lane = lane_default;
     try {
       build_op_device_data(o);
       if (mm.fine) {
@@ -491,7 +486,6 @@ mpdg_status mpdg_op_set_schedule(mpdg_op *op, int precision, const mpdg_schedule
     op->o.sched[precision].cta = sched->cta_cell_groups ? 1 : 0;
     if (sched->lane_cells < 0 || sched->lane_cells > 2) throw Error{MPDG_ERR_ARG, "lane_cells must be 0, 1 or 2"};
     op->o.sched[precision].lane = sched->lane_cells;
-    op->o.sched[precision].band = false;
     return MPDG_OK;
   });
 }

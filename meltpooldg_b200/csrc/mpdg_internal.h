@@ -178,8 +178,9 @@ struct ApplySchedule {
   int evict_first = 0;  // L2 evict-first hint on the coefficient stream
   int pdl = 1;          // colour launches as programmatic dependents of the previous one
   int cta = 0;          // cell groups of a whole CTA (Q2, Q4) instead of a warp
-  int lane = 0;         // Q1, Q2 on uniform lattices, constant coefficients: the band apply
-  bool band = true;     // the band apply wherever it serves the operator (off once a schedule is set)
+  // 0: the coloured launches as above; 1: the band apply or the two launches of a small
+  // mesh where they are faster; 2: the band apply wherever it is built
+  int lane = 1;
 };
 
 struct Op {

@@ -2186,6 +2186,7 @@ bool local_apply_ready(Op &op, const KP<Real> &k)
   const Mesh &m = *op.mesh;
   const long values = m.n_cells * m.n * m.n * m.n;
   if (k.hsrc || k.nvec > 1 || k.zhi > k.zlo || op.local_slot < 0) return false;
+  if (!op.sched[sizeof(Real) == 4 ? MPDG_FP32 : MPDG_FP64].lane) return false;
   if (!m.mapped && (m.nc[0] > 1) + (m.nc[1] > 1) + (m.nc[2] > 1) < 2) return false;  // two colours at most
   if (m.mapped ? !m.d_touch : values > local_values<Real>(op)) return false;
   if (!op.fields_frozen) {
@@ -2409,12 +2410,11 @@ bool band_pays(const Op &op)
   return P == 3 ? fill >= 0.43 && values > 250000 : fill >= 0.65 && values > 500000;
 }
 
-// whether the schedule of one precision runs it: by default where it is faster, and
-// for degrees 1 and 2 where lane_cells asks for it
+// whether the schedule of one precision runs it
 bool band_scheduled(const Op &op, int precision)
 {
-  const ApplySchedule &s = op.sched[precision];
-  return band_serves(op) && (s.band ? band_pays(op) : (s.lane && op.mesh->degree <= 2));
+  const int lane = op.sched[precision].lane;
+  return lane && band_serves(op) && (lane == 2 || band_pays(op));
 }
 
 // element matrices of degree p on [0,1]: mass, stiffness, advection
@@ -3358,7 +3358,7 @@ void autotune_apply(Op &op, int precision, int reps, ApplySchedule &best, double
       for (int d = 0; d <= 1; ++d) {
         for (int g = 0; g <= (cta_differs ? 1 : 0); ++g) {
           ApplySchedule c;
-          c.band = false;
+          c.lane = 0;
           c.slabs = S;
           c.evict_first = h;
           c.pdl = d;
@@ -3367,7 +3367,6 @@ void autotune_apply(Op &op, int precision, int reps, ApplySchedule &best, double
         }
         for (int l = 1; l <= lane_max; ++l) {
           ApplySchedule c;
-          c.band = false;
           c.slabs = S;
           c.evict_first = h;
           c.pdl = d;

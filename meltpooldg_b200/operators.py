@@ -266,10 +266,11 @@ class _MatrixFreeOperator:
         slab by slab over `slabs` z-slabs of cell layers, the L2 evict-first
         hint on the coefficient stream, colour launches that overlap the
         previous colour's tail (programmatic dependent launch), cell groups
-        shared by a whole CTA (degrees 2 and 4), and the band apply
-        (lane_cells 1 or 2: uniform lattices of degree 1 or 2, the default
-        there).  Results do not depend on it, except for rounding with
-        lane_cells."""
+        shared by a whole CTA (degrees 2 and 4); lane_cells 0 takes these
+        coloured launches, 1 (an operator's default) the band apply or the two
+        launches of a small mesh where they are faster, 2 the band apply
+        wherever it is built.  Results do not depend on it, except for rounding
+        where the band apply runs."""
         s = A.Schedule(int(slabs), int(bool(l2_evict_first)), int(bool(overlap_colours)), int(bool(cta_cell_groups)),
                        int(lane_cells))
         A.check(A.lib().mpdg_op_set_schedule(self._h, A.FP32 if precision == "fp32" else A.FP64, C.byref(s)),

@@ -198,3 +198,52 @@ def test_mapped_q1_in_two_launches_where_its_colours_are_many(cuda, n, order, co
     s = dev(rng(4).uniform(-1, 1, gm.n_dofs))
     d = torch.empty_like(s)
     assert launches(lambda: op.vmult(d, s)) == count
+
+
+@pytest.mark.parametrize("p,nc,perturb", [(1, (9, 8, 7), 0.0), (2, (40, 9, 8), 0.0), (3, (20, 20, 10), 0.0),
+                                          (4, (13, 20, 16), 0.0), (2, (9, 8, 7), 0.1), (4, (5, 4, 3), 0.1)])
+def test_setting_the_reported_schedule_changes_nothing(cuda, p, nc, perturb):
+    """get, set: the same launches and bits; lane_cells 0: the coloured launches."""
+    import torch
+    import meltpooldg_b200 as M
+    gm, _ = meshes(nc, p, perturb, seed=3)
+    op = M.HeatDiffuseOperator(gm, 1e-3, precisions=("fp64", "fp32"))
+    for prec, dtype in (("fp64", torch.float64), ("fp32", torch.float32)):
+        s = dev(rng(4).uniform(-1, 1, gm.n_dofs), dtype)
+        a, b = torch.empty_like(s), torch.empty_like(s)
+        default = launches(lambda: op.vmult(a, s))
+        assert default == (2 if perturb else 1)
+        sc = op.schedule(prec)
+        op.set_schedule(precision=prec, **sc)
+        assert op.schedule(prec) == sc
+        assert launches(lambda: op.vmult(b, s)) == default
+        assert torch.equal(a, b)
+        op.set_schedule(precision=prec, **dict(sc, lane_cells=0))
+        assert launches(lambda: op.vmult(b, s)) == 8
+        if perturb:
+            assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("p,nc", [(3, (19, 3, 4)), (3, (20, 9, 2)), (4, (13, 2, 3)), (4, (14, 5, 3)), (4, (1, 9, 2)),
+                                  (2, (1, 1, 9)), (1, (1, 3, 70))])
+@pytest.mark.parametrize("vel", ["none", "const", "rotation"])
+def test_band_apply_wherever_it_is_built(cuda, p, nc, vel):
+    """lane_cells 2 on lattices that the default gives to the other launches."""
+    import torch
+    import meltpooldg_b200 as M
+    v, ov = {"none": (None, {}), "const": ((0.7, -0.4, 0.25), dict(vel_kind=O.VEL_CONST, vel_param=(0.7, -0.4, 0.25))),
+             "rotation": (("rotation", 0.8), dict(vel_kind=O.VEL_ROTATION, vel_param=(0.8, 0.0, 0.0)))}[vel]
+    m = M.boundary_mask(nc, p, faces=[(0, 1), (2, 0)])
+    gm, om = meshes(nc, p, 0.0, mask=m, hi=(1.0, 0.8, 1.3))
+    op = M.AdvectionDiffusionOperator(gm, 1e-3, theta=0.5, diffusivity=1e-2, velocity=v, precisions=("fp64", "fp32"))
+    oop = O.Operator(O.ADVDIFF, 1e-3, theta=0.5, diffusivity=1e-2, dirichlet=m, **ov)
+    src = rng(70 + p).uniform(-1, 1, gm.n_dofs)
+    ref = O.vmult(om, oop, src)
+    for prec, dtype, tol in (("fp64", torch.float64, 1e-12), ("fp32", torch.float32, 2e-5)):
+        op.set_schedule(1, False, prec, overlap_colours=True, lane_cells=2)
+        s = dev(src, dtype)
+        out = torch.full_like(s, float("nan"))
+        if not (p == 4 and vel == "rotation"):
+            assert launches(lambda: op.vmult(out, s)) == 1
+        op.vmult(out, s)
+        assert relerr(out.cpu().numpy().astype(np.float64), ref) < tol
