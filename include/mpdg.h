@@ -312,9 +312,10 @@ typedef struct {
 mpdg_status mpdg_op_set_schedule(mpdg_op *op, int precision, const mpdg_schedule *schedule);
 mpdg_status mpdg_op_get_schedule(mpdg_op *op, int precision, mpdg_schedule *schedule);
 /* Autotuner of the resident apply: times `reps` applies (after one warm-up) of
- * each candidate schedule -- the operator's own first, then slabs 1 and 2, each with
- * and without the evict-first hint where the mesh streams coefficients, each with
- * and without overlap_colours, cta_cell_groups and lane_cells where they apply -- in the given
+ * each candidate schedule -- the operator's own first, the default if that is
+ * another, then the coloured launches in 1 and 2 slabs, each with and without
+ * the evict-first hint where the mesh streams coefficients, overlap_colours and
+ * cta_cell_groups (degrees 2 and 4 on lattices) -- in the given
  * precision (MPDG_FP64 / MPDG_FP32), keeps the fastest on the operator and
  * returns it with its time per apply.  candidate_ms (may be NULL) receives up to
  * n_candidate_ms per-candidate times in that order (-1 past the last).

@@ -252,11 +252,7 @@ mpdg_status mpdg_op_create(mpdg_mesh *mesh, const mpdg_op_desc *desc, mpdg_op **
     o.mesh = &mm;
     o.d = *desc;
     if (o.d.precision_mask == 0) o.d.precision_mask = 1 << MPDG_FP64;
-    // CTA-wide cell groups measured faster for Q2 (both precisions) and Q4 in
-    // FP64 on a B200 (128^3 Q2: 0.664 -> 0.638 ms FP64, 0.399 -> 0.390 ms FP32;
-    // 64^3 Q4 FP64 0.490 -> 0.485 ms; Q4 FP32 0.294 -> 0.299 ms, kept on warps)
-    o.sched[MPDG_FP64].cta = (mm.degree == 2 || mm.degree == 4) ? 1 : 0;
-    o.sched[MPDG_FP32].cta = mm.degree == 2 ? 1 : 0;
+    for (const int prec : {MPDG_FP64, MPDG_FP32}) o.sched[prec] = default_schedule(mm.degree, prec);
     try {
       build_op_device_data(o);
       if (mm.fine) {

@@ -181,7 +181,21 @@ struct ApplySchedule {
   // 0: the coloured launches as above; 1: the band apply or the two launches of a small
   // mesh where they are faster; 2: the band apply wherever it is built
   int lane = 1;
+  bool operator==(const ApplySchedule &o) const
+  {
+    return slabs == o.slabs && evict_first == o.evict_first && pdl == o.pdl && cta == o.cta && lane == o.lane;
+  }
 };
+
+// CTA-wide cell groups measured faster for Q2 (both precisions) and Q4 in
+// FP64 on a B200 (128^3 Q2: 0.664 -> 0.638 ms FP64, 0.399 -> 0.390 ms FP32;
+// 64^3 Q4 FP64 0.490 -> 0.485 ms; Q4 FP32 0.294 -> 0.299 ms, kept on warps)
+inline ApplySchedule default_schedule(int degree, int precision)
+{
+  ApplySchedule s;
+  s.cta = (degree == 2 || (degree == 4 && precision == MPDG_FP64)) ? 1 : 0;
+  return s;
+}
 
 struct Op {
   Mesh *mesh = nullptr;

@@ -3341,21 +3341,19 @@ void autotune_apply(Op &op, int precision, int reps, ApplySchedule &best, double
   const size_t esz = precision == MPDG_FP32 ? sizeof(float) : sizeof(double);
   const size_t bytes = esz * (size_t)m.N;
   reps = std::max(1, reps);
-  // candidates: slabs 1, 2, 4, 8, 16 (as many as the layers allow), each with and
-  // without the evict-first hint where a coefficient stream exists
-  std::vector<ApplySchedule> cand;
-  cand.push_back(op.sched[precision]);  // as the operator stands: by default the fastest known apply
+  // candidates: the operator's schedule, the default (the band apply or two launches
+  // where they are faster) if that is another, then the coloured launches in 1 and 2
+  // slabs, each with and without overlap, CTA cell groups (degrees 2 and 4) and, where a
+  // coefficient stream exists, the evict-first hint
+  std::vector<ApplySchedule> cand{op.sched[precision]};
+  const ApplySchedule def = default_schedule(m.degree, precision);
+  if (!(def == cand[0])) cand.push_back(def);
   const bool stream = !m.uniform || m.mapped;
   const bool cta_differs = (m.degree == 2 || m.degree == 4) && !m.mapped && !op.fine;
-  // the lane apply: uniform lattices of degree 1 or 2 whose vmult takes the
-  // constant-coefficient path with an in-kernel velocity
-  const bool lane_ok = m.uniform && !m.mapped && !op.fine && (m.degree == 1 || m.degree == 2) &&
-                       plain_warp_apply(op) && !uses_kT(op) && op.d.vel_kind != MPDG_VEL_NODAL;
-  const int lane_max = lane_ok && band_serves(op) ? 1 : 0;
   for (int S : {1, 2}) {
     if (S > 1 && (S > m.nc[2] / 2 || m.mapped || op.fine)) continue;
     for (int h = 0; h <= (stream ? 1 : 0); ++h)
-      for (int d = 0; d <= 1; ++d) {
+      for (int d = 0; d <= 1; ++d)
         for (int g = 0; g <= (cta_differs ? 1 : 0); ++g) {
           ApplySchedule c;
           c.lane = 0;
@@ -3363,17 +3361,8 @@ void autotune_apply(Op &op, int precision, int reps, ApplySchedule &best, double
           c.evict_first = h;
           c.pdl = d;
           c.cta = g;
-          cand.push_back(c);
+          if (!(c == cand[0])) cand.push_back(c);
         }
-        for (int l = 1; l <= lane_max; ++l) {
-          ApplySchedule c;
-          c.slabs = S;
-          c.evict_first = h;
-          c.pdl = d;
-          c.lane = l;
-          cand.push_back(c);
-        }
-      }
   }
   void *x = nullptr, *y = nullptr;
   cudaEvent_t e0 = nullptr, e1 = nullptr;

@@ -247,3 +247,21 @@ def test_band_apply_wherever_it_is_built(cuda, p, nc, vel):
             assert launches(lambda: op.vmult(out, s)) == 1
         op.vmult(out, s)
         assert relerr(out.cpu().numpy().astype(np.float64), ref) < tol
+
+
+@pytest.mark.parametrize("p,nc,perturb,count,best", [(2, (40, 9, 8), 0.0, 9, 1), (3, (20, 20, 10), 0.0, 5, 1),
+                                                     (2, (9, 8, 7), 0.1, 17, 2)])
+def test_autotuner_times_each_form_once_and_finds_the_default_again(cuda, p, nc, perturb, count, best):
+    """From the default schedule, and from one that took the coloured launches."""
+    import meltpooldg_b200 as M
+    gm, _ = meshes(nc, p, perturb, seed=3)
+    op = M.HeatDiffuseOperator(gm, 1e-3)
+    s = dev(rng(4).uniform(-1, 1, gm.n_dofs))
+    d = s.clone()
+    sc, _, times = op.autotune("fp64", reps=20)
+    assert len(times) == count and sc["lane_cells"] == 1
+    op.set_schedule(precision="fp64", **dict(sc, lane_cells=0))
+    assert launches(lambda: op.vmult(d, s)) == 8
+    sc, _, times = op.autotune("fp64", reps=20)
+    assert len(times) == count and sc["lane_cells"] == 1
+    assert launches(lambda: op.vmult(d, s)) == best
