@@ -239,9 +239,12 @@ struct Op {
   // small lattices: the cells' results of one apply, before they are gathered; one
   // buffer per stream that the operator was set to (a further stream has none and
   // takes the coloured launches, which need no workspace), FP64-sized, kept in
-  // place until the operator goes
+  // place until the operator goes.  The first one lies behind another array of the
+  // operator (local_spare until a stream takes it), so that it costs no allocation.
   static constexpr int kLocalStreams = 4;
   void *d_local[kLocalStreams] = {};
+  bool local_owned[kLocalStreams] = {};
+  void *local_spare = nullptr;
   cudaStream_t local_stream[kLocalStreams] = {};
   int local_streams = 1;       // slots given out; slot 0 is the default stream's
   int local_slot = 0;          // of the stream set last; -1: none left

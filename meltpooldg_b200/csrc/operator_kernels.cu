@@ -1614,6 +1614,35 @@ T *dev_alloc(size_t count, size_t &bytes)
 
 unsigned grid_for(long n, int block) { return (unsigned)((n + block - 1) / block); }
 
+// local values (cells times (degree + 1)^3) of the largest lattice that applies in two
+// launches in any precision or setting
+constexpr long kLocalValuesMost = 900000;
+
+// bytes of the cells' results of a two-launch apply, where the operator can take one
+// and has no room for them yet
+size_t local_room(const Op &op)
+{
+  const Mesh &m = *op.mesh;
+  const long values = m.n_cells * m.n * m.n * m.n;
+  if (op.local_spare || op.hang_NXc || (m.mapped ? !m.d_touch : values > kLocalValuesMost)) return 0;
+  for (void *p : op.d_local)
+    if (p) return 0;
+  return sizeof(double) * (size_t)values;
+}
+
+// an array of the operator with that room behind it: a driver allocation of its own
+// took 0.3 ms, at the first apply
+template <typename T>
+T *dev_alloc_with_room(Op &op, size_t count)
+{
+  const size_t room = local_room(op), bytes = (sizeof(T) * count + 255) / 256 * 256;
+  char *p = dev_alloc<char>(room ? bytes + room : sizeof(T) * count, op.device_bytes);
+  if (room) op.local_spare = p + bytes;
+  return reinterpret_cast<T *>(p);
+}
+
+bool cells_without_stream(const Op &op);
+
 }  // namespace
 
 void build_mesh_device_data(Mesh &m, const uint8_t *host_mask, bool force_general)
@@ -1761,7 +1790,7 @@ void build_op_device_data(Op &op)
   Mesh &m = *op.mesh;
   const int p = m.degree, n = p + 1, n3 = n * n * n;
   const bool want32 = (op.d.precision_mask & (1 << MPDG_FP32)) != 0;
-  op.d_err = dev_alloc<int>(1, op.device_bytes);
+  op.d_err = cells_without_stream(op) ? dev_alloc_with_room<int>(op, 1) : dev_alloc<int>(1, op.device_bytes);
   MPDG_CUDA(cudaMemset(op.d_err, 0, sizeof(int)));
   if (op.d.kind == MPDG_OP_ADVDIFF && op.d.supg) {
     Colour *d_col = nullptr;
@@ -1864,7 +1893,7 @@ void build_nodal_velocity(Op &op)
   const bool want32 = (op.d.precision_mask & (1 << MPDG_FP32)) != 0;
   const size_t count = (size_t)m.n_cells * velb_stride(n);
   if (!op.d_velb64) {
-    op.d_velb64 = dev_alloc<double>(count, op.device_bytes);
+    op.d_velb64 = m.uniform ? dev_alloc_with_room<double>(op, count) : dev_alloc<double>(count, op.device_bytes);
     MPDG_CUDA(cudaMemsetAsync(op.d_velb64, 0, sizeof(double) * count, op.stream));
   }
   if (want32 && !op.d_velb32) {
@@ -2164,8 +2193,8 @@ template <typename Real>
 long local_values(const Op &op)
 {
   const Mesh &m = *op.mesh;
-  if (sizeof(Real) == 4 || m.uniform) return 900000;
-  return !op.fields_frozen ? 550000 : m.degree == 4 ? 600000 : 900000;
+  if (sizeof(Real) == 4 || m.uniform) return kLocalValuesMost;
+  return !op.fields_frozen ? 550000 : m.degree == 4 ? 600000 : kLocalValuesMost;
 }
 // Mapped meshes gather through the inverse of their map; most have more and smaller
 // colours (11 on a refined box, 17-20 where the cells come in no order).  Us, this and
@@ -2198,9 +2227,16 @@ bool local_apply_ready(Op &op, const KP<Real> &k)
     if (st != cudaStreamCaptureStatusNone) return false;
   }
   void *&buf = op.d_local[op.local_slot];
-  if (!buf && !op.no_build && tracked_malloc(&buf, sizeof(double) * (size_t)values) != cudaSuccess) {
-    cudaGetLastError();
-    buf = nullptr;
+  if (!buf) std::swap(buf, op.local_spare);
+  if (!buf && !op.no_build) {
+    const size_t bytes = sizeof(double) * (size_t)values;
+    if (tracked_malloc(&buf, bytes) == cudaSuccess) {
+      op.local_owned[op.local_slot] = true;
+      op.device_bytes += bytes;
+    } else {
+      cudaGetLastError();
+      buf = nullptr;
+    }
   }
   return buf != nullptr;
 }
@@ -2415,6 +2451,13 @@ bool band_scheduled(const Op &op, int precision)
 {
   const int lane = op.sched[precision].lane;
   return lane && band_serves(op) && (lane == 2 || band_pays(op));
+}
+
+// whether applies run cell by cell without a coefficient or velocity stream of the
+// operator's own, which would carry the room of the two-launch apply
+bool cells_without_stream(const Op &op)
+{
+  return op.mesh->uniform && !supg(op) && !uses_kT(op) && op.d.vel_kind != MPDG_VEL_NODAL && !band_scheduled(op, MPDG_FP64);
 }
 
 // element matrices of degree p on [0,1]: mass, stiffness, advection
@@ -2706,7 +2749,7 @@ void ensure_coef(Op &op, bool want32)
   if (op.coef64_ok && (!want32 || op.coef32_ok)) return;
   const size_t count = (size_t)m.n_cells * metric_stride(m.n);
   if (!op.d_coef64) {
-    op.d_coef64 = dev_alloc<double>(count, op.device_bytes);
+    op.d_coef64 = dev_alloc_with_room<double>(op, count);
     MPDG_CUDA(cudaMemsetAsync(op.d_coef64, 0, sizeof(double) * count, op.stream));
   }
   if (want32 && !op.d_coef32) {
@@ -2758,24 +2801,20 @@ bool ensure_field_coef(Op &op)
     MPDG_CUDA(cudaMemGetInfo(&free_bytes, &total));
     if (sizeof(Real) * (count + (field_fluxes(op) ? fcount : 0)) > free_bytes / 4) return false;
   }
-  auto buffer = [&](auto *&p, size_t cnt) {  // padding is copied, never read
-    using R = std::remove_reference_t<decltype(*p)>;
-    if (p) return;
-    p = dev_alloc<R>(cnt, op.device_bytes);
-    MPDG_CUDA(cudaMemsetAsync(p, 0, sizeof(R) * cnt, op.stream));
-  };
+  // one allocation: the coefficients, then the flux values
+  const size_t head = (count + 63) / 64 * 64, cnt = head + (field_fluxes(op) ? fcount : 0);
   Real *coef = nullptr, *flux = nullptr;
-  if constexpr (f32) {
-    buffer(op.d_coef32, count);
-    if (field_fluxes(op)) buffer(op.d_flux32, fcount);
-    coef = op.d_coef32;
-    flux = op.d_flux32;
-  } else {
-    buffer(op.d_coef64, count);
-    if (field_fluxes(op)) buffer(op.d_flux64, fcount);
-    coef = op.d_coef64;
-    flux = op.d_flux64;
-  }
+  auto streams = [&](Real *&c, Real *&f) {
+    if (!c) {
+      c = dev_alloc_with_room<Real>(op, cnt);
+      f = field_fluxes(op) ? c + head : nullptr;
+      MPDG_CUDA(cudaMemsetAsync(c, 0, sizeof(Real) * cnt, op.stream));  // padding is copied, never read
+    }
+    coef = c;
+    flux = f;
+  };
+  if constexpr (f32) streams(op.d_coef32, op.d_flux32);
+  else streams(op.d_coef64, op.d_flux64);
   KP<double> k = base_params<double>(op);
   if (m.uniform) k.metric = nullptr;
   ColourSet cs;

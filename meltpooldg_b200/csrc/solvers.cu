@@ -8,7 +8,9 @@
 
 #include <chrono>
 #include <cmath>
+#include <initializer_list>
 #include <random>
+#include <utility>
 #include <vector>
 
 #include "mpdg_internal.h"
@@ -31,6 +33,10 @@ struct Workspace {
   double *partial = nullptr;  // reduction partials: 128 groups of kRedBlocks
   double *scal = nullptr;     // device scalars (kNScalars) + GMRES dots (128)
   double *host = nullptr;     // pinned host mirror
+  // the allocations that hold the FP64 and the FP32 vectors: one each, as a driver
+  // allocation takes 0.3 ms (first Newton solve of a new law operator, 40x32x24 Q2, with
+  // its streams also in one: 9-10.5 -> 6.2-7.8 ms)
+  char *block64 = nullptr, *block32 = nullptr;
   size_t bytes = 0;
 };
 
@@ -46,24 +52,33 @@ T *walloc(Workspace &w, size_t count)
   return p;
 }
 
+// one allocation for several arrays, each on a 256-byte boundary
+template <typename T>
+char *carve(Workspace &w, std::initializer_list<std::pair<T **, long>> arrays)
+{
+  auto bytes = [](long count) { return (sizeof(T) * (size_t)count + 255) / 256 * 256; };
+  size_t total = 0;
+  for (const auto &a : arrays) total += bytes(a.second);
+  char *const block = walloc<char>(w, total);
+  char *at = block;
+  for (const auto &a : arrays) {
+    *a.first = reinterpret_cast<T *>(at);
+    at += bytes(a.second);
+  }
+  return block;
+}
+
 Workspace &ws64(Op &op)
 {
   if (!op.ws) op.ws = new Workspace();
   Workspace &w = *op.ws;
   const long N = op.mesh->N;
   w.N = N;
-  if (!w.r) {
-    w.r = walloc<double>(w, N);
-    w.z = walloc<double>(w, N);
-    w.p = walloc<double>(w, N);
-    w.Ap = walloc<double>(w, N);
-    w.invd = walloc<double>(w, N);
-    w.cd = walloc<double>(w, N);
-    w.ct = walloc<double>(w, N);
-    w.partial = walloc<double>(w, 128L * kRedBlocks);
-    w.scal = walloc<double>(w, kNScalars + 128);
+  if (!w.block64) {
+    if (!w.host) MPDG_CUDA(tracked_malloc_host(&w.host, sizeof(double) * (kNScalars + 128)));
+    w.block64 = carve<double>(w, {{&w.r, N}, {&w.z, N}, {&w.p, N}, {&w.Ap, N}, {&w.invd, N}, {&w.cd, N}, {&w.ct, N},
+                                  {&w.partial, 128L * kRedBlocks}, {&w.scal, kNScalars + 128}});
     MPDG_CUDA(cudaMemsetAsync(w.scal, 0, sizeof(double) * kNScalars, op.stream));
-    MPDG_CUDA(tracked_malloc_host(&w.host, sizeof(double) * (kNScalars + 128)));
   }
   return w;
 }
@@ -72,16 +87,9 @@ Workspace &ws32(Op &op)
 {
   Workspace &w = ws64(op);
   const long N = op.mesh->N;
-  if (!w.r32) {
-    w.r32 = walloc<float>(w, N);
-    w.z32 = walloc<float>(w, N);
-    w.p32 = walloc<float>(w, N);
-    w.Ap32 = walloc<float>(w, N);
-    w.x32 = walloc<float>(w, N);
-    w.invd32 = walloc<float>(w, N);
-    w.cd32 = walloc<float>(w, N);
-    w.ct32 = walloc<float>(w, N);
-  }
+  if (!w.block32)
+    w.block32 = carve<float>(w, {{&w.r32, N}, {&w.z32, N}, {&w.p32, N}, {&w.Ap32, N}, {&w.x32, N}, {&w.invd32, N},
+                                 {&w.cd32, N}, {&w.ct32, N}});
   return w;
 }
 
@@ -397,6 +405,7 @@ int gmres(Op &op, Workspace &w, const Prec &P, const R *b, R *x, bool x_is_zero,
   R *&VB = gmres_basis<R>(w, cols);
   if (!VB || *cols < m + 1) {
     if (VB) cudaFree(VB);
+    VB = nullptr;
     VB = walloc<R>(w, (size_t)N * (m + 1));
     *cols = m + 1;
   }
@@ -721,11 +730,7 @@ void free_workspace(Op &op)
 {
   if (!op.ws) return;
   Workspace &w = *op.ws;
-  for (void *p : {(void *)w.r, (void *)w.z, (void *)w.p, (void *)w.Ap, (void *)w.invd, (void *)w.cd,
-                  (void *)w.ct, (void *)w.r32, (void *)w.z32, (void *)w.p32, (void *)w.Ap32,
-                  (void *)w.x32, (void *)w.invd32, (void *)w.cd32, (void *)w.ct32, (void *)w.V,
-                  (void *)w.V32,
-                  (void *)w.partial, (void *)w.scal})
+  for (void *p : {(void *)w.block64, (void *)w.block32, (void *)w.V, (void *)w.V32})
     if (p) cudaFree(p);
   if (w.host) cudaFreeHost(w.host);
   delete op.ws;
