@@ -265,6 +265,9 @@ mpdg_status mpdg_op_device_error(mpdg_op *op, int *flag);
  * its copy with the full limit, so results are unchanged.  No reference
  * counterpart (the reference has no device code). */
 mpdg_status mpdg_debug_set_wait_polls(int64_t polls);
+/* test hook: the bytes that the merged streams of one precision may take in this
+ * operator's solves (see mpdg_solve); < 0 restores a quarter of the device memory */
+mpdg_status mpdg_debug_set_stream_limit(mpdg_op *op, int64_t bytes);
 
 /* OperatorMatrixFree::vmult, operator_base.hpp:239-243
  * (heat: source/heat/heat_diffuse_operator.cpp:179-197;
@@ -368,7 +371,13 @@ mpdg_status mpdg_create_rhs_host(mpdg_op *op, double *dst_host, const double *sr
  * residual estimates of modified Gram-Schmidt in exact arithmetic, and applies
  * the operator once more than it iterates in each cycle that converges.  CG
  * tests convergence on the device after every iteration; the report counts
- * the iterations up to the one that converged. */
+ * the iterations up to the one that converged.  Operators whose coefficients
+ * follow their fields in every apply (phase laws, the full tangent, k(T) on
+ * uniform cells) merge them into streams of 7 to 13 values per quadrature point
+ * for the solve, where these take at most a quarter of the device's memory and
+ * can be allocated beside the solver's vectors; else every apply evaluates the
+ * fields, with the same solution to rounding.  Up to 4 GB of them stay with the
+ * operator for its next solve. */
 mpdg_status mpdg_solve(mpdg_op *op, const mpdg_solver_desc *desc, double *x, const double *b,
                        mpdg_solve_report *report);
 /* host-buffer form of mpdg_solve (x_host in/out, b_host in) */

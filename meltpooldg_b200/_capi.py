@@ -141,6 +141,7 @@ def lib():
     L.mpdg_create_rhs_host.argtypes = [vp, dp, dp, dp]
     L.mpdg_op_device_error.argtypes = [vp, C.POINTER(C.c_int)]
     L.mpdg_debug_set_wait_polls.argtypes = [C.c_int64]
+    L.mpdg_debug_set_stream_limit.argtypes = [vp, C.c_int64]
     L.mpdg_vmult.argtypes = [vp, vp, vp]
     L.mpdg_vmult_f32.argtypes = [vp, vp, vp]
     L.mpdg_vmult_multi.argtypes = [vp, C.c_int, C.POINTER(vp), C.POINTER(vp)]

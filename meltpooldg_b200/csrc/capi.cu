@@ -462,6 +462,15 @@ mpdg_status mpdg_vmult(mpdg_op *op, double *dst, const double *src)
   });
 }
 
+mpdg_status mpdg_debug_set_stream_limit(mpdg_op *op, int64_t bytes)
+{
+  return guarded([&]() -> int {
+    if (!op) throw Error{MPDG_ERR_ARG, "null operator"};
+    op->o.stream_limit = bytes;
+    return MPDG_OK;
+  });
+}
+
 mpdg_status mpdg_debug_set_wait_polls(int64_t polls)
 {
   return guarded([&]() -> int {

@@ -235,7 +235,9 @@ struct Op {
   double *d_flux64 = nullptr;
   float *d_flux32 = nullptr;
   bool fields_frozen = false;  // inside a linear solve: the fields do not change
-  bool merge_declined = false;  // that solve's streams would take too much of the free memory
+  // that solve's streams of a precision would take too much memory, or could not be had
+  bool merge_declined[2] = {false, false};
+  int64_t stream_limit = -1;   // bytes those streams may take (< 0: a quarter of the device memory)
   // small lattices: the cells' results of one apply, before they are gathered; one
   // buffer per stream that the operator was set to (a further stream has none and
   // takes the coloured launches, which need no workspace), FP64-sized, kept in
@@ -357,7 +359,7 @@ struct FrozenFields {
   Op &op;
   bool was;
   explicit FrozenFields(Op &o);
-  ~FrozenFields() { op.fields_frozen = was; }
+  ~FrozenFields();
 };
 
 template <typename Real>

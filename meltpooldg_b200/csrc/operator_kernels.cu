@@ -2785,9 +2785,23 @@ bool live_fields(const Op &op)
 // whether such an operator has velocity or Newton flux values beside the coefficients
 bool field_fluxes(const Op &op) { return uses_law(op) || op.d.full_tangent || op.d.vel_kind != MPDG_VEL_NONE; }
 
-// False where the streams would take more than a quarter of the free device memory
-// (the solver's vectors come after them): the solve then evaluates the fields in
-// every apply, which needs no memory per cell.
+// bytes of merged streams that an operator keeps between solves (a mesh whose applies
+// take two launches, with its room behind the streams, is far below it)
+constexpr size_t kStreamsKept = 4000000000;
+
+size_t device_memory()
+{
+  static const size_t total = [] {
+    size_t free_bytes = 0, total_bytes = 0;
+    MPDG_CUDA(cudaMemGetInfo(&free_bytes, &total_bytes));
+    return total_bytes;
+  }();
+  return total;
+}
+
+// False where the streams would take more than a quarter of the device's memory, or do
+// not fit beside what is there: the solve then evaluates the fields in every apply,
+// which needs no memory per cell.  The solver's vectors are allocated before them.
 template <typename Real>
 bool ensure_field_coef(Op &op)
 {
@@ -2796,25 +2810,26 @@ bool ensure_field_coef(Op &op)
   bool &ok = f32 ? op.coef32_ok : op.coef64_ok;
   if (ok) return true;
   const size_t count = (size_t)m.n_cells * metric_stride(m.n), fcount = 2 * (size_t)m.n_cells * velb_stride(m.n);
-  if (f32 ? !op.d_coef32 : !op.d_coef64) {
-    size_t free_bytes = 0, total = 0;
-    MPDG_CUDA(cudaMemGetInfo(&free_bytes, &total));
-    if (sizeof(Real) * (count + (field_fluxes(op) ? fcount : 0)) > free_bytes / 4) return false;
-  }
   // one allocation: the coefficients, then the flux values
   const size_t head = (count + 63) / 64 * 64, cnt = head + (field_fluxes(op) ? fcount : 0);
-  Real *coef = nullptr, *flux = nullptr;
-  auto streams = [&](Real *&c, Real *&f) {
-    if (!c) {
-      c = dev_alloc_with_room<Real>(op, cnt);
-      f = field_fluxes(op) ? c + head : nullptr;
-      MPDG_CUDA(cudaMemsetAsync(c, 0, sizeof(Real) * cnt, op.stream));  // padding is copied, never read
+  Real *&coef = [&]() -> Real *& {
+    if constexpr (f32) return op.d_coef32;
+    else return op.d_coef64;
+  }();
+  if (!coef) {
+    const int64_t limit = op.stream_limit >= 0 ? op.stream_limit : (int64_t)(device_memory() / 4);
+    if ((int64_t)(sizeof(Real) * cnt) > limit) return false;
+    try {
+      coef = dev_alloc_with_room<Real>(op, cnt);
+    } catch (const Error &) {
+      cudaGetLastError();
+      return false;
     }
-    coef = c;
-    flux = f;
-  };
-  if constexpr (f32) streams(op.d_coef32, op.d_flux32);
-  else streams(op.d_coef64, op.d_flux64);
+    MPDG_CUDA(cudaMemsetAsync(coef, 0, sizeof(Real) * cnt, op.stream));  // padding is copied, never read
+  }
+  Real *const flux = field_fluxes(op) ? coef + head : nullptr;
+  if constexpr (f32) op.d_flux32 = flux;
+  else op.d_flux64 = flux;
   KP<double> k = base_params<double>(op);
   if (m.uniform) k.metric = nullptr;
   ColourSet cs;
@@ -2839,9 +2854,10 @@ bool ensure_field_coef(Op &op)
 template <typename Real>
 bool frozen_field_apply(Op &op, KP<Real> k)
 {
-  if (op.merge_declined || op.mesh->N >= (1L << 32)) return false;  // (the warp apply's 32-bit offsets)
+  bool &declined = op.merge_declined[sizeof(Real) == 4 ? MPDG_FP32 : MPDG_FP64];
+  if (declined || op.mesh->N >= (1L << 32)) return false;  // (the warp apply's 32-bit offsets)
   if (!ensure_field_coef<Real>(op)) {
-    op.merge_declined = true;
+    declined = true;
     return false;
   }
   const bool flux = field_fluxes(op);
@@ -3129,8 +3145,28 @@ void launch_robin(Op &op, Real *dst, const Real *src, int mode)
 FrozenFields::FrozenFields(Op &o) : op(o), was(o.fields_frozen)
 {
   if (!was && live_fields(op)) op.coef64_ok = op.coef32_ok = false;
-  if (!was) op.merge_declined = false;
+  if (!was) op.merge_declined[0] = op.merge_declined[1] = false;
   op.fields_frozen = true;
+}
+
+// large streams go back with the solve, which takes far longer than their allocation
+// (4 GB: 12 million Q2 DoFs); smaller ones stay, as a workspace
+FrozenFields::~FrozenFields()
+{
+  op.fields_frozen = was;
+  if (was || !live_fields(op)) return;
+  const Mesh &m = *op.mesh;
+  const size_t per_cell = metric_stride(m.n) + (field_fluxes(op) ? 2 * velb_stride(m.n) : 0);
+  const size_t bytes64 = op.d_coef64 ? sizeof(double) * per_cell * m.n_cells : 0;
+  const size_t bytes32 = op.d_coef32 ? sizeof(float) * per_cell * m.n_cells : 0;
+  if (bytes64 + bytes32 <= kStreamsKept) return;
+  cudaStreamSynchronize(op.stream);
+  cudaFree(op.d_coef64);
+  cudaFree(op.d_coef32);
+  op.d_coef64 = op.d_flux64 = nullptr;
+  op.d_coef32 = op.d_flux32 = nullptr;
+  op.coef64_ok = op.coef32_ok = false;
+  op.device_bytes -= bytes64 + bytes32;
 }
 
 void invalidate_coef(Op &op)

@@ -367,6 +367,23 @@ float *&gmres_basis<float>(Workspace &w, int *&cols)
   return w.V32;
 }
 
+// vectors of a cycle, and the basis that holds them
+int basis_size(int restart) { return restart > 0 ? std::min(restart, 60) : 30; }
+template <typename R>
+R *reserve_basis(Op &op, Workspace &w, int restart)
+{
+  const int m = basis_size(restart);
+  int *cols = nullptr;
+  R *&VB = gmres_basis<R>(w, cols);
+  if (!VB || *cols < m + 1) {
+    if (VB) cudaFree(VB);
+    VB = nullptr;
+    VB = walloc<R>(w, (size_t)op.mesh->N * (m + 1));
+    *cols = m + 1;
+  }
+  return VB;
+}
+
 template <typename R>
 void dot_any(const R *a, const R *b, long n, double *partial, double *out, cudaStream_t s)
 {
@@ -400,15 +417,8 @@ int gmres(Op &op, Workspace &w, const Prec &P, const R *b, R *x, bool x_is_zero,
   const long N = op.mesh->N;
   cudaStream_t s = op.stream;
   V<R> v = vecs(w, (R *)nullptr);
-  const int m = std::max(1, std::min(restart, 60));
-  int *cols = nullptr;
-  R *&VB = gmres_basis<R>(w, cols);
-  if (!VB || *cols < m + 1) {
-    if (VB) cudaFree(VB);
-    VB = nullptr;
-    VB = walloc<R>(w, (size_t)N * (m + 1));
-    *cols = m + 1;
-  }
+  const int m = basis_size(restart);
+  R *const VB = reserve_basis<R>(op, w, restart);
   // H: the Arnoldi Hessenberg; Hr: its Givens-rotated copy (least squares)
   std::vector<double> H((m + 1) * m, 0.0), Hr((m + 1) * m, 0.0), cs(m), sn(m), g(m + 1), y(m);
   DcgsCoef cf;
@@ -619,6 +629,12 @@ int solve(Op &op, const mpdg_solver_desc &d, double *x, const double *b, mpdg_so
   const auto t0 = std::chrono::steady_clock::now();
   const FrozenFields frozen(op);
   Workspace &w = ws64(op);
+  // the vectors before the streams that the first apply may allocate
+  if (d.mixed_precision) ws32(op);
+  if (d.solver != MPDG_SOLVER_CG) {
+    if (d.mixed_precision) reserve_basis<float>(op, w, d.gmres_restart);
+    else reserve_basis<double>(op, w, d.gmres_restart);
+  }
   const long N = op.mesh->N;
   cudaStream_t s = op.stream;
   rep = mpdg_solve_report{};
@@ -647,8 +663,7 @@ int solve(Op &op, const mpdg_solver_desc &d, double *x, const double *b, mpdg_so
     if (d.solver == MPDG_SOLVER_CG)
       status = pcg<double>(op, w, P, b, x, false, rel, abs_tol, max_it, it, res0, res, applies);
     else
-      status = gmres<double>(op, w, P, b, x, false, rel, abs_tol, max_it,
-                             d.gmres_restart > 0 ? d.gmres_restart : 30, it, res0, res, applies);
+      status = gmres<double>(op, w, P, b, x, false, rel, abs_tol, max_it, d.gmres_restart, it, res0, res, applies);
     rep.iterations = it;
   } else {
     Workspace &w32 = ws32(op);
@@ -697,8 +712,7 @@ int solve(Op &op, const mpdg_solver_desc &d, double *x, const double *b, mpdg_so
       // the inner GMRES reads its rhs from r32, which it uses for nothing else
       // (z32 holds the preconditioner's output)
       int st = gmres<float>(op, w32, P, w32.r32, w32.x32, true, inner, 0.0,
-                            std::max(1, max_it - total), d.gmres_restart > 0 ? d.gmres_restart : 30,
-                            it, r0i, ri, applies);
+                            std::max(1, max_it - total), d.gmres_restart, it, r0i, ri, applies);
       total += it;
       if (st == MPDG_ERR_NAN) {
         status = st;
