@@ -265,3 +265,15 @@ def test_autotuner_times_each_form_once_and_finds_the_default_again(cuda, p, nc,
     sc, _, times = op.autotune("fp64", reps=20)
     assert len(times) == count and sc["lane_cells"] == 1
     assert launches(lambda: op.vmult(d, s)) == best
+
+
+@pytest.mark.parametrize("p", [1, 2, 3, 4])
+def test_default_schedule(cuda, p):
+    """One slab, overlapping colours, CTA cell groups for Q2 and FP64 Q4, the evict-first
+    hint in FP32, the faster form of the apply."""
+    import meltpooldg_b200 as M
+    gm, _ = meshes((3, 3, 3), p, 0.1, seed=3)
+    op = M.HeatDiffuseOperator(gm, 1e-3, precisions=("fp64", "fp32"))
+    common = dict(slabs=1, overlap_colours=True, lane_cells=1)
+    assert op.schedule("fp64") == dict(common, l2_evict_first=False, cta_cell_groups=p in (2, 4))
+    assert op.schedule("fp32") == dict(common, l2_evict_first=True, cta_cell_groups=p == 2)
