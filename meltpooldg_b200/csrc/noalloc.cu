@@ -119,7 +119,7 @@ int solve_cg_noalloc(Op &op, double *x, const double *b, double rel_tol, double 
   if (!std::isfinite(res0)) status = MPDG_ERR_NAN;
   else if (res0 > tol) {
     dev_mul<double>(N, invd, r, z, s);
-    dev_dot(r, z, N, partial, sc + kRZ, s, sc + kTICKET);
+    dev_dot(r, z, N, partial, sc + kRZNEW, s, sc + kTICKET);
     dev_copy<double>(N, z, p, s);
     // the convergence test on the device after every iteration, read every 4
     // iterations (updates past convergence are skipped: results and counts
@@ -131,7 +131,7 @@ int solve_cg_noalloc(Op &op, double *x, const double *b, double rel_tol, double 
       const int batch = std::min(K, max_it - launched);
       for (int bi = 0; bi < batch; ++bi) {
         launch_apply<double>(op, Ap, p);
-        dev_dot(p, Ap, N, partial, sc + kPAP, s, sc + kTICKET);
+        dev_dot(p, Ap, N, partial, sc + kPAP, s, sc + kTICKET, sc);
         dev_cg_update_lagged<double, double>(N, sc, x, r, p, Ap, invd, z, partial, s);
         ++launched;
         dev_cg_direction_lagged<double>(N, sc, p, z, s);

@@ -168,13 +168,19 @@ int pcg(Op &op, Workspace &w, const Prec &P, const R *b, R *x, bool x_is_zero, d
   const double tol = std::fmax(abs_tol, rel_tol * res0);
   if (res0 <= tol) return MPDG_OK;
   prec_apply<R>(op, P, v, v.r, v.z, applies);
-  auto dot_into = [&](const R *a, const R *bb, double *out) {
+  const int K = (N <= (4L << 20)) ? 4 : 1;  // iterations to a host test, see below
+  // Sums end in their kernel's last block, which costs a fence and a ticket per block, or in
+  // a kernel of one block, which costs a launch.  In a replayed graph a launch is the
+  // cheaper of the two for large vectors (CG + Jacobi, us: 118k DoFs 1,205 with tickets,
+  // 1,310 without, 389k 3,175, 3,170, 531k 4,315, 4,190, 1.8M 13,140, 12,850).
+  double *const ticket = K > 1 && N > 400000 ? nullptr : sc + kTICKET;
+  auto dot_into = [&](const R *a, const R *bb, double *out, double *shift = nullptr) {
     if (sizeof(R) == 8)
-      dev_dot((const double *)a, (const double *)bb, N, w.partial, out, s, sc + kTICKET);
+      dev_dot((const double *)a, (const double *)bb, N, w.partial, out, s, ticket, shift);
     else
-      dev_dot_f((const float *)a, (const float *)bb, N, w.partial, out, s, sc + kTICKET);
+      dev_dot_f((const float *)a, (const float *)bb, N, w.partial, out, s, ticket, shift);
   };
-  dot_into(v.r, v.z, sc + kRZ);
+  dot_into(v.r, v.z, sc + kRZNEW);
   dev_copy<R>(N, v.z, v.p, s);
   const bool fused_jacobi = P.kind == MPDG_PREC_JACOBI;
   // The test |r| <= tol runs on the device after every iteration
@@ -183,7 +189,6 @@ int pcg(Op &op, Workspace &w, const Prec &P, const R *b, R *x, bool x_is_zero, d
   // convergence, whose updates are skipped (x, r, p stay those of the
   // converged iteration: the result, the iteration count and the residual are
   // the per-iteration test's).
-  const int K = (N <= (4L << 20)) ? 4 : 1;
   dev_cg_check_init(sc, tol, s);
   const int applies0 = applies;
   int prec_count = 0, launched = 0;
@@ -194,8 +199,8 @@ int pcg(Op &op, Workspace &w, const Prec &P, const R *b, R *x, bool x_is_zero, d
   auto run_batch = [&](int batch) {
     for (int bi = 0; bi < batch; ++bi) {
       launch_apply<R>(op, v.Ap, v.p);
-      dot_into(v.p, v.Ap, sc + kPAP);
-      dev_cg_update_lagged<R, R>(N, sc, x, v.r, v.p, v.Ap, fused_jacobi ? v.invd : nullptr, v.z, w.partial, s);
+      dot_into(v.p, v.Ap, sc + kPAP, sc);
+      dev_cg_update_lagged<R, R>(N, sc, x, v.r, v.p, v.Ap, fused_jacobi ? v.invd : nullptr, v.z, w.partial, s, ticket);
       if (!fused_jacobi) {
         int pa = 0;
         prec_apply<R>(op, P, v, v.r, v.z, pa);
@@ -321,14 +326,12 @@ int pcg_reliable(Op &op, Workspace &w, const Prec &P, const double *b, double *x
   };
   precondition();
   dev_copy<float>(N, v.z, v.p, s);
-  // rz <- rz_new
-  MPDG_CUDA(cudaMemcpyAsync(sc + kRZ, sc + kRZNEW, sizeof(double), cudaMemcpyDeviceToDevice, s));
   double rmax = 1.0;  // iterated residual at the last true residual, scaled
   const bool fused_jacobi = P.kind == MPDG_PREC_JACOBI;
   while (true) {
     launch_apply<float>(op, v.Ap, v.p);
     ++applies;
-    dev_dot_f(v.p, v.Ap, N, w.partial, sc + kPAP, s, sc + kTICKET);
+    dev_dot_f(v.p, v.Ap, N, w.partial, sc + kPAP, s, sc + kTICKET, sc);
     dev_cg_update<float, double>(N, sc, x, v.r, v.p, v.Ap, fused_jacobi ? v.invd : nullptr, v.z,
                                  w.partial, s, scale);
     ++iters;
@@ -574,14 +577,14 @@ double lanczos_lmax(Op &op, Workspace &w, int steps, int &applies)
   dev_copy<double>(N, start, r, s);
   dev_mul<double>(N, w.invd, r, z, s);
   dev_copy<double>(N, z, p, s);
-  dev_dot(r, z, N, w.partial, sc + kRZ, s, sc + kTICKET);
+  dev_dot(r, z, N, w.partial, sc + kRZNEW, s, sc + kTICKET);
   std::vector<double> al, be;
   double *xdummy = w.ct;
   MPDG_CUDA(cudaMemsetAsync(xdummy, 0, sizeof(double) * N, s));
   for (int k = 0; k < steps; ++k) {
     launch_apply<double>(op, Ap, p);
     ++applies;
-    dev_dot(p, Ap, N, w.partial, sc + kPAP, s, sc + kTICKET);
+    dev_dot(p, Ap, N, w.partial, sc + kPAP, s, sc + kTICKET, sc);
     dev_cg_update<double, double>(N, sc, xdummy, r, p, Ap, w.invd, z, w.partial, s);
     MPDG_CUDA(cudaMemcpyAsync(w.host, sc, sizeof(double) * 4, cudaMemcpyDeviceToHost, s));
     MPDG_CUDA(cudaStreamSynchronize(s));

@@ -45,8 +45,7 @@ __device__ __forceinline__ double block_sum(double v)
 // before the call (by thread 0) are then visible to it, and all their threads have
 // read what they read before the call (the last block may overwrite the scalars).  The ticket counts the
 // blocks and is back at 0 afterwards; kernels of one stream may share it.  The last
-// block takes the place of a second launch that read the partials: at 36k DoFs a
-// CG iteration was 9 kernels of 2-4 us each and is 4 now.
+// block takes the place of a second launch that reads the partials.
 __device__ __forceinline__ bool last_block(double *ticket)
 {
   __shared__ bool last;
@@ -60,11 +59,11 @@ __device__ __forceinline__ bool last_block(double *ticket)
   return last;
 }
 
-// sum of the grid's partials (valid in thread 0)
-__device__ __forceinline__ double partial_sum(const double *partial)
+// sum of `blocks` partials (valid in thread 0)
+__device__ __forceinline__ double partial_sum(const double *partial, int blocks)
 {
   double s = 0.0;
-  for (int i = threadIdx.x; i < (int)gridDim.x; i += kRedThreads) s += __ldcg(partial + i);
+  for (int i = threadIdx.x; i < blocks; i += kRedThreads) s += __ldcg(partial + i);
   return block_sum(s);
 }
 
@@ -74,10 +73,12 @@ __device__ __forceinline__ double partial_sum(const double *partial)
 // order, so reductions do not depend on kU.
 constexpr int kU = 4;
 
-// partials of a.b; with a ticket the last block adds them into *out
+// partials of a.b; with a ticket the last block adds them into *out, and (given the
+// scalars of a CG iteration) makes r.z of the last update the one before
 template <typename A, typename B>
 __global__ void __launch_bounds__(kRedThreads) dot_partial_kernel(const A *a, const B *b, long n,
-                                                                  double *partial, double *ticket, double *out)
+                                                                  double *partial, double *ticket, double *out,
+                                                                  double *shift)
 {
   double s = 0.0;
   const long stride = (long)gridDim.x * blockDim.x;
@@ -97,8 +98,11 @@ __global__ void __launch_bounds__(kRedThreads) dot_partial_kernel(const A *a, co
   s = block_sum(s);
   if (threadIdx.x == 0) partial[blockIdx.x] = s;
   if (ticket && last_block(ticket)) {
-    const double t = partial_sum(partial);
-    if (threadIdx.x == 0) *out = t;
+    const double t = partial_sum(partial, gridDim.x);
+    if (threadIdx.x == 0) {
+      *out = t;
+      if (shift) shift[kRZ] = shift[kRZNEW];
+    }
   }
 }
 
@@ -121,8 +125,9 @@ __global__ void __launch_bounds__(kRedThreads) linf_partial_kernel(const double 
 
 // sums (or max-reduces) `count` groups of kRedBlocks partials into out[0..count)
 __global__ void __launch_bounds__(kRedThreads) finish_kernel(const double *partial, int count,
-                                                             double *out, int use_max)
+                                                             double *out, int use_max, double *shift = nullptr)
 {
+  if (shift && threadIdx.x == 0) shift[kRZ] = shift[kRZNEW];
   const int g = blockIdx.x;
   if (g >= count) return;
   double s = 0.0;
@@ -300,7 +305,7 @@ __device__ __forceinline__ void cg_check(double *s)
 // CG step part 1: alpha = s[RZ] / s[PAP]; x += alpha p; r -= alpha Ap;
 // with jacobi: z = invd r; partials of r.r (slot 0) and r.z (slot 1), which the
 // last block adds into s[RR] and s[RZNEW]; it then (LAG) runs the convergence test
-template <typename R, typename RX, bool LAG = false>
+template <typename R, typename RX, bool LAG = false, bool TICKET = true>
 __global__ void __launch_bounds__(kRedThreads) cg_update_kernel(long n, double *s, RX *x,
                                                                 R *r, const R *p, const R *Ap,
                                                                 const R *invd, R *z,
@@ -345,9 +350,9 @@ __global__ void __launch_bounds__(kRedThreads) cg_update_kernel(long n, double *
     rz = block_sum(rz);
     if (threadIdx.x == 0) partial[kRedBlocks + blockIdx.x] = rz;
   }
-  if (!last_block(s + kTICKET)) return;
-  rr = partial_sum(partial);
-  if (invd) rz = partial_sum(partial + kRedBlocks);
+  if (!TICKET || !last_block(s + kTICKET)) return;
+  rr = partial_sum(partial, gridDim.x);
+  if (invd) rz = partial_sum(partial + kRedBlocks, gridDim.x);
   if (threadIdx.x == 0) {
     s[kRR] = rr;
     if (invd) s[kRZNEW] = rz;
@@ -355,9 +360,23 @@ __global__ void __launch_bounds__(kRedThreads) cg_update_kernel(long n, double *
   }
 }
 
-// CG step part 2: beta = s[RZNEW] / s[RZ]; p = z + beta p; s[RZ] <- s[RZNEW] (last block)
+// what the last block of a (LAG) update does, for one without a ticket
+__global__ void __launch_bounds__(kRedThreads) cg_update_finish_kernel(double *s, const double *partial, int blocks, int jacobi)
+{
+  if (s[kDONE] != 0.0) return;
+  const double rr = partial_sum(partial, blocks);
+  const double rz = jacobi ? partial_sum(partial + kRedBlocks, blocks) : 0.0;
+  if (threadIdx.x == 0) {
+    s[kRR] = rr;
+    if (jacobi) s[kRZNEW] = rz;
+    cg_check(s);
+  }
+}
+
+// CG step part 2: beta = s[RZNEW] / s[RZ]; p = z + beta p.  The dot p.Ap that follows
+// makes s[RZNEW] the next s[RZ].
 template <typename R, bool LAG = false>
-__global__ void cg_direction_kernel(long n, double *s, R *p, const R *z)
+__global__ void cg_direction_kernel(long n, const double *s, R *p, const R *z)
 {
   if (LAG && s[kDONE] != 0.0) return;
   const double beta = s[kRZNEW] / s[kRZ];
@@ -374,7 +393,6 @@ __global__ void cg_direction_kernel(long n, double *s, R *p, const R *z)
     for (int u = 0; u < kU; ++u) p[i + u * stride] = (R)((double)vz[u] + beta * (double)vp[u]);
   }
   for (; i < n; i += stride) p[i] = (R)((double)z[i] + beta * (double)p[i]);
-  if (last_block(s + kTICKET) && threadIdx.x == 0) s[kRZ] = s[kRZNEW];
 }
 
 // Chebyshev start: d = invd r / theta; z = d
@@ -465,22 +483,29 @@ unsigned red_blocks(long n)
 }
 }  // namespace
 
-void dev_dot(const double *a, const double *b, long n, double *partial, double *out, cudaStream_t s, double *ticket)
+namespace {
+template <typename R>
+void dot_any(const R *a, const R *b, long n, double *partial, double *out, cudaStream_t s, double *ticket, double *shift)
 {
-  dot_partial_kernel<double, double><<<ticket ? red_blocks(n) : kRedBlocks, kRedThreads, 0, s>>>(a, b, n, partial, ticket, out);
+  dot_partial_kernel<R, R><<<ticket ? red_blocks(n) : kRedBlocks, kRedThreads, 0, s>>>(a, b, n, partial, ticket, out, shift);
   MPDG_LAUNCHED();
   if (ticket) return;
-  finish_kernel<<<1, kRedThreads, 0, s>>>(partial, 1, out, 0);
+  finish_kernel<<<1, kRedThreads, 0, s>>>(partial, 1, out, 0, shift);
   MPDG_LAUNCHED();
 }
 
-void dev_dot_f(const float *a, const float *b, long n, double *partial, double *out, cudaStream_t s, double *ticket)
+}  // namespace
+
+void dev_dot(const double *a, const double *b, long n, double *partial, double *out, cudaStream_t s, double *ticket,
+             double *shift)
 {
-  dot_partial_kernel<float, float><<<ticket ? red_blocks(n) : kRedBlocks, kRedThreads, 0, s>>>(a, b, n, partial, ticket, out);
-  MPDG_LAUNCHED();
-  if (ticket) return;
-  finish_kernel<<<1, kRedThreads, 0, s>>>(partial, 1, out, 0);
-  MPDG_LAUNCHED();
+  dot_any<double>(a, b, n, partial, out, s, ticket, shift);
+}
+
+void dev_dot_f(const float *a, const float *b, long n, double *partial, double *out, cudaStream_t s, double *ticket,
+               double *shift)
+{
+  dot_any<float>(a, b, n, partial, out, s, ticket, shift);
 }
 
 void dev_linf(const double *a, long n, double *partial, double *out, cudaStream_t s)
@@ -572,8 +597,7 @@ template <typename R, typename RX>
 void dev_cg_update(long n, double *s, RX *x, R *r, const R *p, const R *Ap, const R *invd, R *z,
                    double *partial, cudaStream_t st, double xscale)
 {
-  cg_update_kernel<R, RX><<<red_blocks(n), kRedThreads, 0, st>>>(n, s, x, r, p, Ap, invd, z, partial,
-                                                              xscale);
+  cg_update_kernel<R, RX><<<red_blocks(n), kRedThreads, 0, st>>>(n, s, x, r, p, Ap, invd, z, partial, xscale);
   MPDG_LAUNCHED();
 }
 template void dev_cg_update<double, double>(long, double *, double *, double *, const double *,
@@ -597,17 +621,24 @@ template void dev_cg_direction<float>(long, double *, float *, const float *, cu
 
 template <typename R, typename RX>
 void dev_cg_update_lagged(long n, double *s, RX *x, R *r, const R *p, const R *Ap, const R *invd, R *z,
-                          double *partial, cudaStream_t st)
+                          double *partial, cudaStream_t st, bool ticket)
 {
-  cg_update_kernel<R, RX, true><<<red_blocks(n), kRedThreads, 0, st>>>(n, s, x, r, p, Ap, invd, z, partial, 1.0);
+  if (ticket) {
+    cg_update_kernel<R, RX, true><<<red_blocks(n), kRedThreads, 0, st>>>(n, s, x, r, p, Ap, invd, z, partial, 1.0);
+    MPDG_LAUNCHED();
+    return;
+  }
+  cg_update_kernel<R, RX, true, false><<<kRedBlocks, kRedThreads, 0, st>>>(n, s, x, r, p, Ap, invd, z, partial, 1.0);
+  MPDG_LAUNCHED();
+  cg_update_finish_kernel<<<1, kRedThreads, 0, st>>>(s, partial, kRedBlocks, invd != nullptr);
   MPDG_LAUNCHED();
 }
 template void dev_cg_update_lagged<double, double>(long, double *, double *, double *, const double *,
                                                    const double *, const double *, double *, double *,
-                                                   cudaStream_t);
+                                                   cudaStream_t, bool);
 template void dev_cg_update_lagged<float, float>(long, double *, float *, float *, const float *,
                                                  const float *, const float *, float *, double *,
-                                                 cudaStream_t);
+                                                 cudaStream_t, bool);
 
 template <typename R>
 void dev_cg_direction_lagged(long n, double *s, R *p, const R *z, cudaStream_t st)

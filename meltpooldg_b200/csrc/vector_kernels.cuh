@@ -17,11 +17,12 @@ enum { kDONE = 4, kCONV = 5, kRRCONV = 6, kTOL = 7 };
 // block ticket of the reductions that finish in their last block (zero between kernels)
 enum { kTICKET = 15 };
 
-// a.b into *out: by a second kernel, or in the last block given a zeroed ticket
+// a.b into *out: by a second kernel, or in the last block given a zeroed ticket.  Given the scalars of a CG iteration as `shift`, s[kRZ] <- s[kRZNEW] too: a
+// direction has been formed since the update.
 void dev_dot(const double *a, const double *b, long n, double *partial, double *out, cudaStream_t s,
-             double *ticket = nullptr);
+             double *ticket = nullptr, double *shift = nullptr);
 void dev_dot_f(const float *a, const float *b, long n, double *partial, double *out, cudaStream_t s,
-               double *ticket = nullptr);
+               double *ticket = nullptr, double *shift = nullptr);
 void dev_linf(const double *a, long n, double *partial, double *out, cudaStream_t s);
 // delayed classical Gram-Schmidt (GMRES): the dots V_k.u and, when w is given,
 // V_k.w for k < m (out[k], out[m + k]), one pass over the basis
@@ -57,7 +58,7 @@ void dev_cg_direction(long n, double *s, R *p, const R *z, cudaStream_t st);
 // (|r| <= s[kTOL], or r.r not finite)
 template <typename R, typename RX>
 void dev_cg_update_lagged(long n, double *s, RX *x, R *r, const R *p, const R *Ap, const R *invd, R *z,
-                          double *partial, cudaStream_t st);
+                          double *partial, cudaStream_t st, bool ticket = true);
 template <typename R>
 void dev_cg_direction_lagged(long n, double *s, R *p, const R *z, cudaStream_t st);
 // resets the state slots and sets the tolerance
