@@ -2446,11 +2446,15 @@ bool band_pays(const Op &op)
   return P == 3 ? fill >= 0.43 && values > 250000 : fill >= 0.65 && values > 500000;
 }
 
-// whether the schedule of one precision runs it
-bool band_scheduled(const Op &op, int precision)
+// whether the schedule of one precision runs it.  An apply over a range of layers has no
+// two-launch form to give small lattices to: one launch a range instead of eight
+// (mpdg_vmult_host of 4x4x500 Q2 cells in eight ranges 85 us, 220)
+bool band_scheduled(const Op &op, int precision, bool range = false)
 {
+  const Mesh &m = *op.mesh;
   const int lane = op.sched[precision].lane;
-  return lane && band_serves(op) && (lane == 2 || band_pays(op));
+  return lane && band_serves(op) &&
+         (lane == 2 || band_pays(op) || (range && m.n_cells * m.n * m.n * m.n <= kLocalValuesMost));
 }
 
 // whether applies run cell by cell without a coefficient or velocity stream of the
@@ -2662,7 +2666,7 @@ template <typename Real, int GEOM>
 void warp_apply_degree(Op &op, const KP<Real> &k)
 {
   if constexpr (GEOM == GEOM_UNIFORM) {
-    if (band_scheduled(op, sizeof(Real) == 4 ? MPDG_FP32 : MPDG_FP64)) {
+    if (band_scheduled(op, sizeof(Real) == 4 ? MPDG_FP32 : MPDG_FP64, k.zhi > k.zlo)) {
       band_apply<Real>(op, k);
       return;
     }

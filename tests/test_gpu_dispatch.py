@@ -277,3 +277,15 @@ def test_default_schedule(cuda, p):
     common = dict(slabs=1, overlap_colours=True, lane_cells=1)
     assert op.schedule("fp64") == dict(common, l2_evict_first=False, cta_cell_groups=p in (2, 4))
     assert op.schedule("fp32") == dict(common, l2_evict_first=True, cta_cell_groups=p == 2)
+
+
+@pytest.mark.parametrize("p,nc", [(2, (4, 4, 60)), (4, (5, 4, 20)), (3, (9, 8, 17))])
+def test_host_pipeline_of_small_lattices_takes_one_launch_a_range(cuda, p, nc):
+    """Eight ranges of layers (as many as pairs of layers allow), one launch each."""
+    import meltpooldg_b200 as M
+    gm, om = meshes(nc, p, 0.0)
+    op = M.HeatDiffuseOperator(gm, 1e-3)
+    src = rng(4).uniform(-1, 1, gm.n_dofs)
+    out = np.empty_like(src)
+    assert launches(lambda: op.vmult_host(out, src)) == 8
+    assert relerr(out, O.vmult(om, O.Operator(O.HEAT, 1e-3), src)) < 1e-12
