@@ -2184,7 +2184,8 @@ int num_sms()
 // coloured apply's, bit for bit.  Measured, us, this and coloured (general cells unless
 // said otherwise), below and above the lines:
 //   FP64        Q1 40^3 (512k values) 15, 23   Q4 4x4x300 (600k) 20.5, 20-22  Q2 30^3 (729k) 22.6, 19.6
-//   FP64 uniform, velocity vector              Q4 4x4x300 18.6, 22.5          Q2 2x128x128 (885k) 22.6, 22.6
+//   FP64 uniform                               Q3 24^3 (885k) 20.6, 22.6      Q4 19^3 (857k) 22.7, 22.9
+//   with a velocity vector                     Q4 17^3 (614k) 20.6, 22.8      Q4 18^3 (729k) 27.1, 23.9
 //   FP32        Q4 4x16x100 (800k) 18.6, 22.1  Q2 2x128x128 20.4, 22.2        Q4 25^3 (1.95M) 37, 30
 // Within a solve an apply follows another kernel of 3-8 us, and a round trip in GMRES, so
 // two launches pay for longer: Newton step of Q2 gas/liquid/solid heat at 829k values
@@ -2193,7 +2194,8 @@ template <typename Real>
 long local_values(const Op &op)
 {
   const Mesh &m = *op.mesh;
-  if (sizeof(Real) == 4 || m.uniform) return kLocalValuesMost;
+  if (sizeof(Real) == 4) return kLocalValuesMost;
+  if (m.uniform) return m.degree == 4 && op.d.vel_kind == MPDG_VEL_NODAL ? 650000 : kLocalValuesMost;
   return !op.fields_frozen ? 550000 : m.degree == 4 ? 600000 : kLocalValuesMost;
 }
 // Mapped meshes gather through the inverse of their map; most have more and smaller
@@ -3579,7 +3581,7 @@ void launch_rhs(Op &op, double *dst, const double *src, const double *heat_sourc
     k.full_tangent = 0;
     // SUPG: + tau_K u (phi_old/dt - (1-theta) u.grad phi_old + (1-theta) D lap phi_old)
     // tested with grad N (advection_diffusion_operator.cpp:336-346)
-    // 128^3 Q2 vortex: 1,600 us by the block kernel in eight colours, 200 as line products;
+    // 64^3 Q2 vortex: 213 us by the block kernel in eight colours, 52 as line products;
     // not on strips that are nearly empty, us, line products and cells: Q2 1x1x4000
     // (share 0.02) 24, 15, 4x4x4000 (0.11) 46, 80; Q3 4x4x4000 (0.16) 186, 131, 4x4000x4
     // (0.20) 96, 131; Q4 4x4x4000 (0.23) 425, 249, 4x4000x4 (0.29) 204, 247

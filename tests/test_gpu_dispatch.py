@@ -13,19 +13,36 @@ pytestmark = pytest.mark.gpu
 SLACK = 1.5
 
 
-def best_us(f, n=20, batches=7):
+def best_us(*calls, n=20, batches=9):
+    """Best time of each call, batches in turn."""
     import torch
-    f()
-    torch.cuda.synchronize()
-    e0, e1, best = torch.cuda.Event(True), torch.cuda.Event(True), float("inf")
+    e0, e1, best = torch.cuda.Event(True), torch.cuda.Event(True), [float("inf")] * len(calls)
+    for f in calls:
+        f()
     for _ in range(batches):
-        e0.record()
-        for _ in range(n):
-            f()
-        e1.record()
-        torch.cuda.synchronize()
-        best = min(best, 1e3 * e0.elapsed_time(e1) / n)
+        for i, f in enumerate(calls):
+            torch.cuda.synchronize()
+            e0.record()
+            for _ in range(n):
+                f()
+            e1.record()
+            torch.cuda.synchronize()
+            best[i] = min(best[i], 1e3 * e0.elapsed_time(e1) / n)
     return best
+
+
+def colours(op, p):
+    """The default schedule's coloured launches."""
+    op.set_schedule(1, False, "fp64", overlap_colours=True, cta_cell_groups=p in (2, 4), lane_cells=0)
+    return op
+
+
+def launches(f):
+    import meltpooldg_b200 as M
+    f()
+    before = M.kernel_launches()
+    f()
+    return M.kernel_launches() - before
 
 
 def coloured(op, dst, src):
@@ -61,26 +78,34 @@ def test_two_launches_on_thin_lattices_are_not_slower_than_the_colours(cuda, p, 
     import torch
     import meltpooldg_b200 as M
     gm, _ = meshes(nc, p, 0.1, seed=3)
-    op = M.HeatDiffuseOperator(gm, 1e-3)
+    op, ref = M.HeatDiffuseOperator(gm, 1e-3), colours(M.HeatDiffuseOperator(gm, 1e-3), p)
     s = dev(rng(4).uniform(-1, 1, gm.n_dofs))
     d = torch.empty_like(s)
-    two = best_us(lambda: op.vmult(d, s))
-    eight = best_us(coloured(op, d, s).replay)
+    two, eight = best_us(lambda: op.vmult(d, s), lambda: ref.vmult(d, s))
     assert two < SLACK * eight, (two, eight)
 
 
-def test_long_lattices_are_not_slower_than_the_colours(cuda):
-    """4,000 cell layers: what the host does for one launch does not grow with them."""
+def test_host_time_of_an_apply_does_not_grow_with_the_layers(cuda):
+    """The band apply's search for its chunks on 4,000 cell layers against 40."""
+    import time
     import torch
     import meltpooldg_b200 as M
-    gm, _ = meshes((2, 2, 4000), 1, 0.0)
-    op = M.HeatDiffuseOperator(gm, 1e-3)
-    s = dev(rng(4).uniform(-1, 1, gm.n_dofs))
-    d = torch.empty_like(s)
-    default = best_us(lambda: op.vmult(d, s))
-    op.set_schedule(1, False, "fp64", overlap_colours=True, lane_cells=0)
-    eight = best_us(coloured(op, d, s).replay)
-    assert default < SLACK * eight, (default, eight)
+    host = []
+    for nz in (40, 4000):
+        gm, _ = meshes((16, 4, nz), 1, 0.0)
+        op = M.HeatDiffuseOperator(gm, 1e-3)
+        s = dev(rng(4).uniform(-1, 1, gm.n_dofs))
+        d = torch.empty_like(s)
+        assert launches(lambda: op.vmult(d, s)) == 1
+        best = float("inf")
+        for _ in range(30):
+            torch.cuda.synchronize()
+            t = time.perf_counter()
+            for _ in range(5):
+                op.vmult(d, s)
+            best = min(best, time.perf_counter() - t)
+        host.append(best)
+    assert host[1] < 2.5 * host[0], host
 
 
 @pytest.mark.parametrize("p,nc,vel", [(4, (8, 60, 40), ("rotation", 0.8)), (4, (24, 24, 24), ("rotation", 0.8)),
@@ -93,12 +118,11 @@ def test_the_default_apply_is_not_slower_than_the_colours(cuda, p, nc, vel):
     import torch
     import meltpooldg_b200 as M
     gm, _ = meshes(nc, p, 0.0)
-    op = M.AdvectionDiffusionOperator(gm, 1e-3, theta=0.5, diffusivity=1e-2, velocity=vel)
+    op, ref = (M.AdvectionDiffusionOperator(gm, 1e-3, theta=0.5, diffusivity=1e-2, velocity=vel) for _ in range(2))
+    colours(ref, p)
     s = dev(rng(4).uniform(-1, 1, gm.n_dofs))
     d, e = torch.empty_like(s), torch.empty_like(s)
-    default = best_us(lambda: op.vmult(d, s))
-    op.set_schedule(1, False, "fp64", overlap_colours=True, cta_cell_groups=p in (2, 4), lane_cells=0)
-    eight = best_us(coloured(op, e, s).replay)
+    default, eight = best_us(lambda: op.vmult(d, s), lambda: ref.vmult(e, s))
     assert (d - e).abs().max() <= 1e-13 * e.abs().max()
     assert default < SLACK * eight, (default, eight)
 
@@ -137,7 +161,7 @@ def test_diagonal_from_line_factors_is_not_slower_than_from_the_cells(cuda, p, n
         gm, _ = meshes(nc, p, 0.0, geometry=geometry)
         op = M.AdvectionDiffusionOperator(gm, 1e-3, theta=0.5, diffusivity=1e-2, velocity=vel)
         d.append(torch.empty(gm.n_dofs, dtype=torch.float64, device="cuda"))
-        us.append(best_us(lambda: op.compute_diagonal(d[-1])))
+        us += best_us(lambda: op.compute_diagonal(d[-1]))
     assert (d[0] - d[1]).abs().max() <= 1e-12 * d[1].abs().max()
     assert us[0] < SLACK * us[1], us
 
@@ -155,26 +179,28 @@ def test_rhs_as_line_products_is_not_slower_than_from_the_cells(cuda, p, nc):
         d.append(torch.zeros(gm.n_dofs, dtype=torch.float64, device="cuda"))
         op.create_rhs(d[-1], phi)
         spare = torch.zeros_like(phi)
-        us.append(best_us(lambda: op.create_rhs(spare, phi)))
+        us += best_us(lambda: op.create_rhs(spare, phi))
     assert (d[0] - d[1]).abs().max() <= 1e-12 * d[1].abs().max()
     assert us[0] < SLACK * us[1], us
 
 
-def launches(f):
-    import meltpooldg_b200 as M
-    f()
-    before = M.kernel_launches()
-    f()
-    return M.kernel_launches() - before
-
-
 def test_two_launches_up_to_the_measured_sizes(cuda):
-    """General cells: FP64 up to 550,000 local values outside a solve, FP32 up to 900,000."""
+    """General cells: FP64 up to 550,000 local values outside a solve, FP32 up to 900,000;
+    uniform Q4 cells with a velocity vector: FP64 up to 650,000."""
     import torch
     import meltpooldg_b200 as M
     for nc, fp64 in (((28, 28, 24), 2), ((32, 32, 24), 8)):
         gm, _ = meshes(nc, 2, 0.1, seed=3)
         op = M.HeatDiffuseOperator(gm, 1e-3, precisions=("fp64", "fp32"))
+        for dtype, n in ((torch.float64, fp64), (torch.float32, 2)):
+            s = dev(rng(4).uniform(-1, 1, gm.n_dofs), dtype)
+            d = torch.empty_like(s)
+            assert launches(lambda: op.vmult(d, s)) == n
+    for nc, fp64 in (((17, 17, 17), 2), ((18, 18, 18), 8)):
+        gm, _ = meshes(nc, 4, 0.0)
+        op = M.AdvectionDiffusionOperator(gm, 1e-3, theta=0.5, diffusivity=1e-2, velocity="nodal", precisions=("fp64", "fp32"))
+        U = dev(rng(5).uniform(-1, 1, 3 * gm.n_dofs))
+        op.set_velocity(U)
         for dtype, n in ((torch.float64, fp64), (torch.float32, 2)):
             s = dev(rng(4).uniform(-1, 1, gm.n_dofs), dtype)
             d = torch.empty_like(s)
