@@ -379,19 +379,26 @@ struct ColourRuns {
   }
 };
 
+// DoFs of a small lattice (N^2 < 2^40) and magic divisors of its NX and NY
+struct GatherDivs {
+  unsigned N;
+  unsigned long long mx, my;
+};
+
 // dst from the cells' local results: a DoF adds the values of its cells in the order
 // of their colours, as the coloured launches do, so the bits are the same;
 // constrained DoFs get 0.  A thread per DoF of the flattened lattice: a block per 128
 // of a row left 123 of 128 threads idle on rows of 5 DoFs (apply of general Q2 cells
 // 2 x 128 x 128, FP64: 82 us, in colours 23, so 27; Q1 2 x 200 x 200: 60, 23, 17)
 template <int P, typename Real>
-__global__ void __launch_bounds__(128) local_gather_kernel(const KP<Real> p, const ColourRuns runs, unsigned N)
+__global__ void __launch_bounds__(128) local_gather_kernel(const KP<Real> p, const ColourRuns runs, const GatherDivs d)
 {
   constexpr int n = P + 1, n2 = n * n, n3 = n2 * n;
   const unsigned at = blockIdx.x * blockDim.x + threadIdx.x, NX = (unsigned)p.NX, NY = (unsigned)p.NY;
-  const bool in = at < N;
-  const unsigned g = in ? at : 0, row = g / NX;
-  const int X = (int)(g - row * NX), Z = (int)(row / NY), Y = (int)(row - (unsigned)Z * NY);
+  const bool in = at < d.N;
+  const unsigned g = in ? at : 0, row = (unsigned)((g * d.mx) >> 40);
+  const unsigned Zu = (unsigned)((row * d.my) >> 40);
+  const int X = (int)(g - row * NX), Z = (int)Zu, Y = (int)(row - Zu * NY);
   const bool masked = in && p.masked_write && p.dmask && p.dmask[g];
   // per axis and parity: the cell of that parity that has the node, and the node in it
   int cx[2], lx[2], cy[2], ly[2], cz[2], lz[2];

@@ -2287,6 +2287,9 @@ void run_local_apply(Op &op, KP<Real> k)
   // the gather starts as the cells' CTAs retire and waits before its first read
   cudaLaunchConfig_t cfg = {};
   const long N = MAPPED ? m.N : m.NX * m.NY * m.NZ;
+  constexpr unsigned long long two40 = 1ull << 40;
+  if (!MAPPED && (unsigned long long)N * (unsigned long long)N >= two40) throw Error{MPDG_ERR_SIZE, "gather index arithmetic"};
+  const GatherDivs divs{(unsigned)N, (two40 + m.NX - 1) / std::max(1L, m.NX), (two40 + m.NY - 1) / std::max(1L, m.NY)};
   cfg.gridDim = dim3(grid_for(N, 128));
   cfg.blockDim = dim3(128);
   cfg.stream = op.stream;
@@ -2299,7 +2302,7 @@ void run_local_apply(Op &op, KP<Real> k)
     MPDG_CUDA(cudaLaunchKernelEx(&cfg, mapped_gather_kernel<Real>, k.dst, (const Real *)k.local, (const int *)m.d_touch_ptr,
                                  (const int *)m.d_touch, k.masked_write ? k.dmask : nullptr, N));
   else
-    MPDG_CUDA(cudaLaunchKernelEx(&cfg, local_gather_kernel<P, Real>, k, runs, (unsigned)N));
+    MPDG_CUDA(cudaLaunchKernelEx(&cfg, local_gather_kernel<P, Real>, k, runs, divs));
   MPDG_LAUNCHED();
 }
 
