@@ -2435,10 +2435,13 @@ double strip_fill(const Mesh &m)
 //   Q4 0.65  9x28x49 (0.62) 31, 28         19x34x50 (0.66) 51, 56     64^3 235, 397
 // Small lattices are latency: at degrees 1 and 2 one launch is sooner than two down to a
 // share of 0.03 (Q1 4x100x4 4.9, 8.2, Q2 6x45x11 6.2, 8.2; single cells in x and y, Q2
-// 1x1x1000 vortex 14, 7); at degrees 3 and 4 a plane of a strip takes 2 us (Q3 16^3 12.3,
-// 10.3, 20^3 12.3, 15.1; Q4 16^3 20.5, 17.2, 10x10x60 21.3, 24.6).  The rotation at
-// degree 3 (576 bytes of spills): 40^3 (0.65) 53, 52, 1000x4x4 26, 23, 45x39x52 (0.73)
-// 59, 71, 64^3 146, 189.
+// 1x1x1000 vortex 14, 7).  At degrees 3 and 4 a plane of a strip takes 2 us: columns of
+// single cells go to their two colours (Q3 1000x1x1 10.3, 7.6), flat Q4 lattices to two
+// launches (100x4x4 22.6, 10.3); elsewhere one launch needs no room for local results,
+// whose allocation (0.3 ms) the two would have to earn back first (Q3 16^3 12.3, 10.3,
+// 20^3 12.3, 15.1; Q4 16^3 20.5, 17.2, 10x10x60 21.3, 24.6; eight colours 19-23).  The
+// rotation at degree 3 (576 bytes of spills): 40^3 (0.65) 53, 52, 1000x4x4 26, 23,
+// 45x39x52 (0.73) 59, 71, 64^3 146, 189.
 bool band_pays(const Op &op)
 {
   const Mesh &m = *op.mesh;
@@ -2448,7 +2451,8 @@ bool band_pays(const Op &op)
   if (P == 3 && op.d.vel_kind == MPDG_VEL_ROTATION) return fill >= 0.70 && m.nc[1] >= 16 && values > 1500000;
   if (P == 1) return fill >= (values <= 100000 ? 0.03 : 0.08);
   if (P == 2) return fill >= (values <= 100000 ? 0.03 : 0.20);
-  return P == 3 ? fill >= 0.43 && values > 250000 : fill >= 0.65 && values > 500000;
+  if ((m.nc[0] > 1) + (m.nc[1] > 1) + (m.nc[2] > 1) < 2) return false;
+  return P == 3 ? fill >= 0.43 : fill >= 0.65 && (m.nc[1] >= 8 || values > 500000);
 }
 
 // whether the schedule of one precision runs it.  An apply over a range of layers has no

@@ -111,7 +111,8 @@ def test_host_time_of_an_apply_does_not_grow_with_the_layers(cuda):
 @pytest.mark.parametrize("p,nc,vel", [(4, (8, 60, 40), ("rotation", 0.8)), (4, (24, 24, 24), ("rotation", 0.8)),
                                       (3, (2, 100, 100), None), (4, (2, 100, 100), None), (3, (4, 16, 500), None),
                                       (2, (4, 4, 4000), ("rotation", 0.8)), (1, (4, 16, 4000), "vortex"),
-                                      (4, (1, 1, 100), None), (3, (30, 1, 1), ("rotation", 0.8))])
+                                      (4, (1, 1, 100), None), (3, (30, 1, 1), ("rotation", 0.8)),
+                                      (3, (1000, 1, 1), None)])
 def test_the_default_apply_is_not_slower_than_the_colours(cuda, p, nc, vel):
     """Uniform lattices whose strips of the band apply would stay nearly empty, or whose
     products spill: the default takes the launches that are faster there."""
@@ -129,7 +130,7 @@ def test_the_default_apply_is_not_slower_than_the_colours(cuda, p, nc, vel):
 
 @pytest.mark.parametrize("p,nc", [(3, (20, 20, 10)), (3, (19, 3, 70)), (4, (13, 20, 16)), (4, (27, 10, 16))])
 @pytest.mark.parametrize("mask", ["none", "some_faces", "scattered"])
-def test_band_apply_of_degrees_3_and_4_at_its_smallest_sizes(cuda, p, nc, mask):
+def test_band_apply_of_degrees_3_and_4(cuda, p, nc, mask):
     import torch
     import meltpooldg_b200 as M
     m = {"none": lambda: None, "some_faces": lambda: M.boundary_mask(nc, p, faces=[(0, 1), (2, 0)]),
