@@ -2181,22 +2181,21 @@ int num_sms()
 // Small lattices apply in two launches -- all cells into local results, then a
 // gather per DoF -- instead of eight colours, whose launches take 19-23 us whatever the
 // size; the extra pass over n^3 values per cell stays in the L2.  The sums are the
-// coloured apply's, bit for bit.  Measured, us, this and coloured (general cells unless
-// said otherwise), below and above the lines:
-//   FP64        Q1 40^3 (512k values) 15, 23   Q4 4x4x300 (600k) 20.5, 20-22  Q2 30^3 (729k) 22.6, 19.6
-//   FP64 uniform                               Q3 24^3 (885k) 20.6, 22.6      Q4 19^3 (857k) 22.7, 22.9
-//   with a velocity vector                     Q4 17^3 (614k) 20.6, 22.8      Q4 18^3 (729k) 27.1, 23.9
-//   FP32        Q4 4x16x100 (800k) 18.6, 22.1  Q2 2x128x128 20.4, 22.2        Q4 25^3 (1.95M) 37, 30
-// Within a solve an apply follows another kernel of 3-8 us, and a round trip in GMRES, so
-// two launches pay for longer: Newton step of Q2 gas/liquid/solid heat at 829k values
-// 3.94 ms, 4.08; CG Q2 829k 6.11, 6.12, Q3 682k 6.6, 7.2; but Q4 512k 7.1, 7.4, 729k 8.8, 8.5.
+// coloured apply's, bit for bit.  Measured, us, this and coloured, with the operands of
+// three operators in turn (as a time step meets them), below the line and above it:
+//   FP64 general   Q1 45^3 (729k) 20.2, 21.4   Q2 32^3 (885k) 24.8, 27.4   Q3 24^3 24.2, 26.0   Q4 19^3 26.1, 27.5
+//   with velocity  Q1 48^3 (885k) 24.7, 26.6   Q2 31^3 (804k) 26.4, 26.4   Q3 24^3 26.7, 28.9   Q4 19^3 28.4, 29.8
+//   FP32 general   Q2 32^3 18.5, 22.4          Q4 19^3 18.6, 23.7          Q4 25^3 (1.95M, one operator) 37, 30
+//   FP64 uniform, velocity vector              Q4 17^3 (614k) 20.6, 22.8   Q4 18^3 (729k) 27.1, 23.9
+// One operator's operands over and over, all in the L2, FP64 general: even at 700k (Q1
+// 18-20, 20, Q2 20, 20), 885k Q2 24.6, 21.6.  Within a solve: Newton step of Q2
+// gas/liquid/solid heat at 829k values 3.94 ms, 4.08; CG Q2 829k 6.1, 6.1, Q3 682k 6.6,
+// 7.2, Q4 729k 8.7, 8.5.
 template <typename Real>
 long local_values(const Op &op)
 {
-  const Mesh &m = *op.mesh;
-  if (sizeof(Real) == 4) return kLocalValuesMost;
-  if (m.uniform) return m.degree == 4 && op.d.vel_kind == MPDG_VEL_NODAL ? 650000 : kLocalValuesMost;
-  return !op.fields_frozen ? 550000 : m.degree == 4 ? 600000 : kLocalValuesMost;
+  const bool q4_vector = op.mesh->uniform && op.mesh->degree == 4 && op.d.vel_kind == MPDG_VEL_NODAL;
+  return sizeof(Real) == 8 && q4_vector ? 650000 : kLocalValuesMost;
 }
 // Mapped meshes gather through the inverse of their map; most have more and smaller
 // colours (11 on a refined box, 17-20 where the cells come in no order).  Us, this and
